@@ -416,50 +416,10 @@ def render_gaussians(background, image_height, image_width, means2D, depths, rad
         if stats is not None:
             ev1.record()
             stats["forward_render_time"] = _EventMs([(ev0, ev1)])
-        _density_copy(geomBuffer, g["records"], P)
         if debug:
             _check_device(dev)
     return (R, out_color, n_render, n_consider, n_contrib, out_observe, out_all_map, out_plane_depth,
             geomBuffer, binningBuffer, imgBuffer)
-
-
-# ---- density hand-over --------------------------------------------------------------------------------------
-# The forward pass measures how densely the splats cover the pixel blocks they touch and leaves the counters behind
-# its records; the backward pass picks its walk from them.  It can do so on the device (both kernels queued, one
-# returns at once).  Cheaper: the counters are copied to pinned memory right behind the forward pass, and if they
-# have arrived by the time the backward pass is queued (they have whenever something else ran in between) the
-# choice is made here and one kernel is launched.  The copy is never waited for.
-_DENSITY = {}
-_density_pinned = None
-_density_next = 0
-_DENSITY_SLOTS = 256
-
-
-def _density_copy(geomBuffer, records, P):
-    global _density_pinned, _density_next
-    n = _lib.lib().cgx_render_density_words()
-    if _density_pinned is None:
-        _density_pinned = torch.zeros(_DENSITY_SLOTS, n, dtype=torch.int64).pin_memory()
-    if len(_DENSITY) >= _DENSITY_SLOTS // 2:
-        _DENSITY.clear()                        # forward passes whose backward never came
-    slot = _density_next
-    _density_next = (_density_next + 1) % _DENSITY_SLOTS
-    _lib.check(_lib.lib().cgx_post_words(C.c_void_p(records.data_ptr() + P * 64),
-                                         C.c_void_p(_density_pinned[slot].data_ptr()), 2 * n, _stream()),
-               "cgx_post_words")
-    ev = torch.cuda.Event()
-    ev.record()
-    _DENSITY[geomBuffer.data_ptr()] = (slot, ev)
-
-
-def _density_walk(geomBuffer):
-    """0: let the device decide; 1: per-pixel lists; 2: every pixel looks at every visit."""
-    hit = _DENSITY.pop(geomBuffer.data_ptr(), None)
-    if hit is None or not hit[1].query():
-        return 0
-    c = _density_pinned[hit[0]]
-    pixels, visits = int(c[0::2].sum()), int(c[1::2].sum())
-    return 2 if pixels > _lib.lib().cgx_render_dense_threshold() * visits else 1
 
 
 def render_gaussians_backward(background, tan_fovx, tan_fovy, all_map_pixels, all_maps, R, geomBuffer, binningBuffer,
@@ -503,7 +463,8 @@ def render_gaussians_backward_2d(background, tan_fovx, tan_fovy, all_map_pixels,
                 ev0 = torch.cuda.Event(enable_timing=True)
                 ev1 = torch.cuda.Event(enable_timing=True)
                 ev0.record()
-            _call("cgx_render_bwd", l.cgx_render_bwd, P, W, H, float(tan_fovx), float(tan_fovy), _ptr(im["ranges"]), _ptr(b["point_list"]),
+            workspace = torch.empty(l.cgx_render_bwd_workspace_bytes(P), dtype=torch.uint8, device=dev)
+            _call("cgx_render_bwd", l.cgx_render_bwd_table, P, W, H, float(tan_fovx), float(tan_fovy), _ptr(im["ranges"]), _ptr(b["point_list"]),
                                    _ptr(_cuda_f32(background, "background")), _ptr(g["records"]),
                                    _ptr(_cuda_f32(all_map_pixels, "all_map_pixels")), _ptr(im["accum_alpha"]),
                                    _ptr(im["n_contrib"]), _ptr(local),
@@ -512,7 +473,8 @@ def render_gaussians_backward_2d(background, tan_fovx, tan_fovy, all_map_pixels,
                                    _ptr(_cuda_f32(dL_dout_plane_depth, "dL_dout_plane_depth")),
                                    int(bool(render_geo)), _ptr(dL_dmeans2D), _ptr(dL_dmeans2D_abs),
                                    _ptr(dL_dconic_opacity), _ptr(dL_dcolors), _ptr(dL_dall_map),
-                                   _density_walk(geomBuffer), st, info=dict(P=P, R=R, HW=H * W, local=local))
+                                   0, _ptr(g["tiles_touched"]), _ptr(workspace), workspace.numel(), st,
+                                   info=dict(P=P, R=R, HW=H * W, local=local))
             if stats is not None:
                 ev1.record()
                 stats["backward_render_time"] = _EventMs([(ev0, ev1)])

@@ -107,6 +107,8 @@ SIGNATURES = {
     "cgx_launch_count": (C.c_uint64, []),
     "cgx_tile_stats": (_i, [_i, _i] + [_vp] * 8),
     "cgx_render_bwd": (_i, [_i, _i, _i, _f, _f] + [_vp] * 11 + [_i] + [_vp] * 5 + [_i, _vp]),
+    "cgx_render_bwd_workspace_bytes": (_sz, [_i]),
+    "cgx_render_bwd_table": (_i, [_i, _i, _i, _f, _f] + [_vp] * 11 + [_i] + [_vp] * 5 + [_i, _vp, _vp, _sz, _vp]),
     "cgx_render_density_words": (_i, []),
     "cgx_render_dense_threshold": (_i, []),
     "cgx_device_status": (_i, [_vp, _vp]),

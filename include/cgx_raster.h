@@ -478,25 +478,37 @@ int cgx_render_bwd(int P, int W, int H, float tanfovx, float tanfovy, const uint
                    float* dL_dmeans2D, float* dL_dmeans2D_abs, float* dL_dconic_opacity, float* dL_drgb,
                    float* dL_dall_map, int walk, void* stream);
 
-/* How the backward pass chooses its walk.  cgx_render_fwd leaves, behind the P records of its `records` buffer,
- * cgx_render_density_words() 64-bit counters: pairs (pixels that passed the alpha test, visits of a Gaussian to an
- * 8x4 pixel block), spread over slots.  walk = 0: cgx_render_bwd queues both of its kernels and the one the
- * counters do not call for returns at once (no host read).  A caller that has the counters on the host anyway
- * (copied behind the forward pass; by the time of the backward pass they have usually arrived) sums the pairs and
- * passes walk = 2 (every pixel looks at every visit) when pixels > cgx_render_dense_threshold() * visits, else
- * walk = 1 (every pixel walks its own list): one launch instead of two. */
+/* The same with a workspace of cgx_render_bwd_workspace_bytes(P) bytes (16-byte aligned, contents irrelevant) and the
+ * tiles_touched (P) that the counting stage wrote: the sums go to one 64-byte row per Gaussian and from there to the
+ * five tensors, instead of with scattered atomics into them.  workspace NULL = cgx_render_bwd. */
+size_t cgx_render_bwd_workspace_bytes(int P);
+int cgx_render_bwd_table(int P, int W, int H, float tanfovx, float tanfovy, const uint32_t* ranges,
+                         const uint32_t* point_list, const float* bg, const void* records,
+                         const float* all_map_pixels, const float* final_T, const uint32_t* n_contrib,
+                         const uint8_t* compute_locally, const float* dL_dcolor, const float* dL_dout_all_map,
+                         const float* dL_dout_plane_depth, int render_geo,
+                         float* dL_dmeans2D, float* dL_dmeans2D_abs, float* dL_dconic_opacity, float* dL_drgb,
+                         float* dL_dall_map, int walk, const uint32_t* tiles_touched, void* workspace, size_t workspace_bytes,
+                         void* stream);
+
+/* Small and large splats.  cgx_render_fwd leaves, behind the P records of its `records` buffer,
+ * cgx_render_density_words() 64-bit counters: pairs (pixels that Gaussians may reach, Gaussians that meet an 8x4 pixel
+ * block), spread over slots.  The backward pass rounds the exponent of alpha one way where pixels >
+ * cgx_render_dense_threshold() * meetings and another way elsewhere (a contribution within an ulp of the 1/255
+ * threshold is kept or dropped accordingly).  walk = 0: by the counters, on the device; a caller that knows passes
+ * walk = 2 (above the threshold) or 1. */
 int cgx_render_density_words(void);
 int cgx_render_dense_threshold(void);
 
 /* ------------------------------------------------------------------ diagnostics */
 
 /* Host-synchronous.  Waits for `stream`, reads and clears the device status word that kernels set when a
- * bounded wait (blending mbarriers, peer barrier, the sort's look-back) gives up (0 = ok, CGX_ETIMEDOUT otherwise).  Replaces the reference's debug-mode
+ * bounded wait (peer barrier, the sort's look-back) gives up (0 = ok, CGX_ETIMEDOUT otherwise).  Replaces the reference's debug-mode
  * synchronise-and-throw (RAST/cuda_rasterizer/auxiliary.h:220-227); nothing ever traps. */
 int cgx_device_status(int* status_host, void* stream);
 
 /* The same status words without waiting: queues their copies on `stream` into status_pinned_host4[0..2]
- * (page-locked host memory: blending kernels, peer barrier, sort look-back; [3] is reserved and set to 0).  The
+ * (page-locked host memory: [1] peer barrier, [2] sort look-back; [0] and [3] are set to 0).  The
  * caller looks at them after a synchronisation it performs anyway (0 = ok); the words are not cleared
  * (cgx_device_status clears them). */
 int cgx_device_status_async(int* status_pinned_host4, void* stream);
