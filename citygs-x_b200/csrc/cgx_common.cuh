@@ -28,6 +28,8 @@ int post_words(const void* src_dev, void* dst_host_pinned, int n_words, cudaStre
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+__device__ __forceinline__ bool aligned16_dev(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
 // Column-major 3x3 (m[c][r]); product order matches the usual column-major definition
 // r[c][row] = a[0][row]*b[c][0] + a[1][row]*b[c][1] + a[2][row]*b[c][2], summed left to right.
 struct Mat3 {
