@@ -7,12 +7,21 @@ screen-space position gradient of the Gaussians that were visible (`radii > 0` f
 of the screen radius.  It is what the benchmark's capacity sweep updates every step.  `AnchorStatistics` is the form
 the reference's trainer actually calls for its anchor model (scene/gaussian_model.py:1181-1205 ``training_statis``).
 
-The reference indexes with boolean masks (a host synchronisation per mask); here every update is a dense masked
-expression, so nothing blocks the host.  Values are identical: rows outside the mask receive +0.
+The reference indexes with boolean masks (a host synchronisation per mask); here nothing blocks the host.  On a GPU
+an update is one or two kernels (`cgx_densify_update`, `cgx_anchor_stats`); elsewhere, and for tensors of other types or
+layouts, a dense masked expression with the same values (rows outside the mask receive +0).
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
+
+MAX_CAMS = 16
+
+
+def _plain(t, dtype):
+    return t.is_cuda and t.dtype == dtype and t.is_contiguous()
 
 
 class DensificationStats:
@@ -36,8 +45,27 @@ class DensificationStats:
 
     def update_batch(self, per_camera):
         """per_camera: iterable of (radii, means2D), e.g. ``TrainingStep.last``."""
-        for radii, means2D in per_camera:
-            self.update(radii, means2D)
+        per_camera = [(r, m.grad, m) for r, m in per_camera if m.grad is not None]
+        P, dev = self.grad_accum.shape[0], self.grad_accum.device
+        fused = P > 0 and _plain(self.grad_accum, torch.float32) and _plain(self.denom, torch.float32) and \
+            (self.max_radii2D is None or _plain(self.max_radii2D, torch.int32)) and \
+            all(_plain(r, torch.int32) and _plain(g, torch.float32) and r.numel() == P and g.shape == (P, 2) and
+                r.device == dev and g.device == dev for r, g, _ in per_camera)
+        if not fused:
+            for radii, _, means2D in per_camera:
+                self.update(radii, means2D)
+            return
+        from diff_gaussian_rasterization import _lib
+
+        with torch.cuda.device(dev):
+            for i in range(0, len(per_camera), MAX_CAMS):
+                part = per_camera[i:i + MAX_CAMS]
+                ptrs = C.c_void_p * len(part)
+                _lib.check(_lib.lib().cgx_densify_update(
+                    P, len(part), ptrs(*[r.data_ptr() for r, _, _ in part]), ptrs(*[g.data_ptr() for _, g, _ in part]),
+                    self.grad_accum.data_ptr(), self.denom.data_ptr(),
+                    None if self.max_radii2D is None else self.max_radii2D.data_ptr(), _lib.current_stream_ptr()),
+                    "cgx_densify_update")
 
     def mean_gradient(self):
         """Average gradient norm over the visits, NaN-free (0 where never visible): what the densifier thresholds."""
@@ -52,7 +80,8 @@ class AnchorStatistics:
     on screen).
 
     The reference writes through chained boolean indexing (`x[mask] += y`, one host synchronisation per mask).
-    Here every update is a ``masked_scatter`` of a dense source, so nothing blocks the host; the values are the same.
+    Here the ranks that chained indexing stands for come from partial counts of the masks inside two kernels; off the
+    GPU every update is a ``masked_scatter`` of a dense source.  The values are the same.
     """
 
     def __init__(self, n_anchors: int, n_offsets: int, device):
@@ -69,6 +98,27 @@ class AnchorStatistics:
         bool, Gaussian was on screen (radii > 0); offset_selection_mask: (V * n_offsets,) bool, slot produced a
         Gaussian (G = its number of True entries); anchor_visible_mask: (N,) bool with V True entries."""
         n_off = self.n_offsets
+        accums = (self.opacity_accum, self.anchor_demon, self.offset_gradient_accum, self.offset_denom)
+        masks = (update_filter, offset_selection_mask, anchor_visible_mask)
+        if all(_plain(t, torch.float32) for t in accums) and all(_plain(m, torch.bool) for m in masks) and \
+                _plain(opacity, torch.float32) and viewspace_point_grad.is_cuda and \
+                viewspace_point_grad.dtype == torch.float32 and viewspace_point_grad.ndim == 2 and \
+                viewspace_point_grad.shape[1] >= 2 and viewspace_point_grad.stride(1) == 1 and \
+                opacity.numel() == offset_selection_mask.numel() and anchor_visible_mask.numel() and \
+                update_filter.numel() == viewspace_point_grad.shape[0] and \
+                len({t.device for t in accums + masks + (opacity, viewspace_point_grad)}) == 1:
+            from diff_gaussian_rasterization import _lib
+
+            l = _lib.lib()
+            N, slots = anchor_visible_mask.numel(), offset_selection_mask.numel()
+            ws = torch.empty(l.cgx_anchor_stats_workspace_bytes(N, slots), dtype=torch.uint8, device=opacity.device)
+            with torch.cuda.device(opacity.device):
+                _lib.check(l.cgx_anchor_stats(
+                    N, n_off, slots, update_filter.numel(), viewspace_point_grad.data_ptr(),
+                    max(2, viewspace_point_grad.stride(0)), opacity.data_ptr(), update_filter.data_ptr(),
+                    offset_selection_mask.data_ptr(), anchor_visible_mask.data_ptr(), *[t.data_ptr() for t in accums],
+                    ws.data_ptr(), ws.numel(), _lib.current_stream_ptr()), "cgx_anchor_stats")
+            return
         avm = anchor_visible_mask.view(-1, 1)
         per_anchor = opacity.detach().reshape(-1).clamp_min(0).view(-1, n_off).sum(dim=1, keepdim=True)
         self.opacity_accum += torch.zeros_like(self.opacity_accum).masked_scatter(avm, per_anchor)

@@ -16,7 +16,7 @@ CSRC = ROOT / "csrc"
 LIBDIR = ROOT / "lib"
 # CGX_RASTER_LIB: load another build of the same library (A/B timing of compile-time tile sizes); never a fallback
 SO = Path(os.environ["CGX_RASTER_LIB"]) if os.environ.get("CGX_RASTER_LIB") else LIBDIR / "libcgx_raster.so"
-SOURCES = ["cabi.cu", "preprocess.cu", "binning.cu", "render.cu", "peer.cu", "loss.cu", "redistribute.cu"]
+SOURCES = ["cabi.cu", "preprocess.cu", "binning.cu", "render.cu", "peer.cu", "loss.cu", "redistribute.cu", "stats.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-shared", "-Xcompiler", "-fPIC"]
 
@@ -109,6 +109,9 @@ SIGNATURES = {
     "cgx_render_bwd": (_i, [_i, _i, _i, _f, _f] + [_vp] * 11 + [_i] + [_vp] * 5 + [_i, _vp]),
     "cgx_render_bwd_workspace_bytes": (_sz, [_i]),
     "cgx_render_bwd_table": (_i, [_i, _i, _i, _f, _f] + [_vp] * 11 + [_i] + [_vp] * 5 + [_i, _vp, _vp, _sz, _vp]),
+    "cgx_densify_update": (_i, [_i, _i] + [_vp] * 6),
+    "cgx_anchor_stats_workspace_bytes": (_sz, [_i, _i64]),
+    "cgx_anchor_stats": (_i, [_i, _i, _i64, _i64, _vp, _i] + [_vp] * 9 + [_sz, _vp]),
     "cgx_render_density_words": (_i, []),
     "cgx_render_dense_threshold": (_i, []),
     "cgx_device_status": (_i, [_vp, _vp]),

@@ -500,6 +500,23 @@ int cgx_render_bwd_table(int P, int W, int H, float tanfovx, float tanfovy, cons
 int cgx_render_density_words(void);
 int cgx_render_dense_threshold(void);
 
+/* ------------------------------------------------------------------ densification statistics */
+
+/* Per Gaussian, over B <= 16 cameras in order: where radii[b] > 0, |dL_dmeans2D[b]| (P,2) is added to grad_accum and 1
+ * to denom; max_radii (optional) takes the largest radius seen.  radii / dL_dmeans2D: HOST arrays of device pointers. */
+int cgx_densify_update(int P, int B, const int32_t* const* radii, const float* const* dL_dmeans2D, float* grad_accum,
+                       float* denom, int32_t* max_radii, void* stream);
+
+/* scene/gaussian_model.py:1181-1205 `training_statis`: bytes 0/1 seen (n_anchors); the V visible anchors own the
+ * n_slots = V * n_offsets slots of opacity / selected (n_slots) in order, the selected slots the n_gaussians rows of
+ * grad (grad_stride >= 2 floats apart, the first two used) and on_screen in order.  Adds to opacity_accum, anchor_demon
+ * (n_anchors), gradient_accum, denom (n_anchors * n_offsets).  What the masks' sums do not support is left out. */
+size_t cgx_anchor_stats_workspace_bytes(int n_anchors, int64_t n_slots);
+int cgx_anchor_stats(int n_anchors, int n_offsets, int64_t n_slots, int64_t n_gaussians, const float* grad,
+                     int grad_stride, const float* opacity, const uint8_t* on_screen, const uint8_t* selected,
+                     const uint8_t* seen, float* opacity_accum, float* anchor_demon, float* gradient_accum, float* denom,
+                     void* workspace, size_t workspace_bytes, void* stream);
+
 /* ------------------------------------------------------------------ diagnostics */
 
 /* Host-synchronous.  Waits for `stream`, reads and clears the device status word that kernels set when a
