@@ -164,7 +164,10 @@ def preprocess_gaussians_batched(means3D, scales, rotations, shs, opacities, ras
     stand-alone op).  ``pipeline`` (a `Pipeline`) splits both launches into chunks of Gaussians so that a caller
     can overlap its host-to-device parameter copies and device-to-host gradient copies with them."""
     settings = list(raster_settings_list)
-    flat = _PreprocessBatched.apply(means3D, scales, rotations, opacities, settings, cuda_args, bool(planes), pipeline)
+    if pipeline is None and _C.PROFILE is None:
+        flat = _lib.host().preprocess_batched(means3D, scales, rotations, opacities, settings, bool(planes))
+    else:       # with a caller's hooks between the chunks, or events around every launch
+        flat = _PreprocessBatched.apply(means3D, scales, rotations, opacities, settings, cuda_args, bool(planes), pipeline)
     rgb = torch.zeros(means3D.shape[0], 3, device=means3D.device)
     n = 5 if planes else 4
     return [(flat[n * b], rgb, flat[n * b + 1], flat[n * b + 2], flat[n * b + 3]) + ((flat[n * b + 4],) if planes else ())

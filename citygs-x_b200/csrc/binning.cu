@@ -33,9 +33,13 @@ analyse_mask_kernel(int gx, int gy, const uint8_t* __restrict__ local, MaskBand*
         s_full = 0;
     }
     __syncthreads();
-    for (int y = threadIdx.x; y < gy; y += blockDim.x) {
+    // a warp per tile row (a thread per row read its bytes one after the other: 5 us at 1920x1080, 10 at 3840x2160)
+    const int lane = threadIdx.x & 31;
+    for (int y = threadIdx.x >> 5; y < gy; y += blockDim.x >> 5) {
         int set = 0;
-        for (int x = 0; x < gx; x++) set += local[y * gx + x] ? 1 : 0;
+        for (int x = lane; x < gx; x += 32) set += local[y * gx + x] ? 1 : 0;
+        set = __reduce_add_sync(0xffffffffu, set);
+        if (lane) continue;
         if (set == gx) {
             atomicMin(&s_first, y);
             atomicMax(&s_last, y);
@@ -217,10 +221,11 @@ __device__ __forceinline__ uint32_t scan_row_inplace(uint32_t* __restrict__ row,
 // block_ranges (optional): per-CTA (min, max) depth bit patterns -> total_out[1], total_out[2].
 __global__ void __launch_bounds__(1024)
 scan_partials_kernel(int n, uint32_t* __restrict__ sums, uint32_t* __restrict__ total_out,
-                     const uint32_t* __restrict__ block_ranges)
+                     const uint32_t* __restrict__ block_ranges, volatile uint32_t* host_words)
 {
     const uint32_t total = scan_row_inplace(sums, n);
     if (threadIdx.x == 0) total_out[0] = total;
+    uint32_t all_min = 0xffffffffu, all_max = 0u;
     if (block_ranges) {
         __shared__ uint32_t s_min[32], s_max[32];
         uint32_t lo = 0xffffffffu, hi = 0u;
@@ -240,9 +245,17 @@ scan_partials_kernel(int n, uint32_t* __restrict__ sums, uint32_t* __restrict__ 
                 lo = min(lo, s_min[w]);
                 hi = max(hi, s_max[w]);
             }
-            total_out[1] = lo;
-            total_out[2] = hi;
+            total_out[1] = all_min = lo;
+            total_out[2] = all_max = hi;
         }
+    }
+    // the host watches the fourth word (see cgx_bin_count_scan_post)
+    if (host_words && threadIdx.x == 0) {
+        host_words[0] = total;
+        host_words[1] = all_min;
+        host_words[2] = all_max;
+        __threadfence_system();
+        host_words[3] = 1u;
     }
 }
 
@@ -1295,10 +1308,15 @@ extern "C" size_t cgx_bin_workspace_bytes(int P)
 
 static int bin_count_scan(int P, int W, int H, const int32_t* radii, const float* means2D, const float* depths,
                           const uint8_t* compute_locally, uint32_t* tiles_touched, uint32_t* num_rendered,
-                          void* workspace, size_t workspace_bytes, void* stream)
+                          void* workspace, size_t workspace_bytes, void* stream, uint32_t* host_words = nullptr)
 {
     if (P < 0 || W <= 0 || H <= 0 || !num_rendered) return CGX_EINVAL;
     cudaStream_t st = (cudaStream_t)stream;
+    void* mapped = nullptr;
+    if (host_words) {       // fails for pageable memory: the caller must pass page-locked memory
+        cudaError_t e = cudaHostGetDevicePointer(&mapped, host_words, 0);
+        if (e != cudaSuccess || !mapped) { (void)cudaGetLastError(); return CGX_EINVAL; }
+    }
     if (P == 0) {
         cudaError_t e = cudaMemsetAsync(num_rendered, 0, (depths ? 3 : 1) * sizeof(uint32_t), st);
         if (e != cudaSuccess) { set_cuda_error(e); return CGX_ECUDA; }
@@ -1316,7 +1334,7 @@ static int bin_count_scan(int P, int W, int H, const int32_t* radii, const float
     const int vec_ok = aligned16(radii) && aligned16(means2D) && aligned16(tiles_touched) && (!depths || aligned16(depths));
     tile_count_kernel<<<nblocks, CGX_BLOCK_SIZE, 0, st>>>(P, gx, gy, radii, (const float2*)means2D, compute_locally,
                                                           tiles_touched, sums, band, depths, block_ranges, vec_ok);
-    scan_partials_kernel<<<1, 1024, 0, st>>>(nblocks, sums, num_rendered, block_ranges);
+    scan_partials_kernel<<<1, 1024, 0, st>>>(nblocks, sums, num_rendered, block_ranges, (volatile uint32_t*)mapped);
     return check_launch(3);
 }
 
@@ -1335,6 +1353,16 @@ extern "C" int cgx_bin_count_scan_depths(int P, int W, int H, const int32_t* rad
     if (P > 0 && !depths) return CGX_EINVAL;
     return bin_count_scan(P, W, H, radii, means2D, depths, compute_locally, tiles_touched, num_rendered3, workspace,
                           workspace_bytes, stream);
+}
+
+extern "C" int cgx_bin_count_scan_post(int P, int W, int H, const int32_t* radii, const float* means2D,
+                                       const float* depths, const uint8_t* compute_locally, uint32_t* tiles_touched,
+                                       uint32_t* num_rendered3, void* workspace, size_t workspace_bytes,
+                                       uint32_t* host_words4, void* stream)
+{
+    if (P <= 0 || !host_words4) return CGX_EINVAL;
+    return bin_count_scan(P, W, H, radii, means2D, depths, compute_locally, tiles_touched, num_rendered3, workspace,
+                          workspace_bytes, stream, host_words4);
 }
 
 extern "C" int cgx_emit_keys(int P, int W, int H, const int32_t* radii, const float* means2D, const float* depths,

@@ -1,0 +1,852 @@
+// Host path of the differentiable operators: checks, allocations, launches and autograd nodes in C++.
+//
+// The Python operators of this package cost about 0.8 ms of interpreter time per camera and training step (ctypes calls,
+// torch.autograd.Function, tensor views of scratch buffers), several times what the kernels of a small step take on the
+// device.  These nodes call the same C ABI (include/cgx_raster.h) through the addresses that Python resolved, so one
+// library serves both; the raw entry points of diff_gaussian_rasterization._C and its per-stage profiling stay in Python.
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/extension.h>
+
+#include <atomic>
+#include <chrono>
+#include <map>
+#include <mutex>
+
+#include "../../include/cgx_raster.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+namespace {
+
+// ---------------------------------------------------------------------------------------------- the library
+#define CGX_FUNCTIONS(X)                                                                                             \
+    X(cgx_preprocess_fwd) X(cgx_preprocess_bwd) X(cgx_preprocess_fwd_batched_planes) X(cgx_preprocess_bwd_batched_planes) \
+    X(cgx_all_map_fwd) X(cgx_all_map_bwd) X(cgx_strip_loss_fwd) X(cgx_strip_loss_bwd) X(cgx_depth_normal_fwd)        \
+    X(cgx_depth_normal_bwd) X(cgx_bin_workspace_bytes) X(cgx_bin_count_scan_post) X(cgx_emit_keys)                   \
+    X(cgx_sort_workspace_bytes) X(cgx_sort_passes) X(cgx_sort_pairs_pingpong) X(cgx_tile_ranges) X(cgx_higher_msb)   \
+    X(cgx_render_records_bytes) X(cgx_render_fwd) X(cgx_render_bwd_workspace_bytes) X(cgx_render_bwd_table)
+struct Library {
+#define X(f) decltype(&::f) f = nullptr;
+    CGX_FUNCTIONS(X)
+#undef X
+} L;
+PyObject* error_class = nullptr;      // _lib.CgxError
+
+void bind(const py::dict& addresses, py::object error)
+{
+#define X(f) L.f = reinterpret_cast<decltype(L.f)>(addresses[#f].cast<uintptr_t>());
+    CGX_FUNCTIONS(X)
+#undef X
+    error_class = error.release().ptr();
+}
+
+void check(int status, const char* where)
+{
+    if (status == CGX_OK) return;
+    py::gil_scoped_acquire gil;
+    py::object e = py::reinterpret_borrow<py::object>(error_class)(status, where);
+    PyErr_SetObject(error_class, e.ptr());
+    throw py::error_already_set();
+}
+
+// ---------------------------------------------------------------------------------------------- small helpers
+Tensor cuda_f32(const Tensor& t, const char* name)
+{
+    if (!t.is_cuda()) throw std::runtime_error(std::string(name) + " must be a CUDA tensor (this rasterizer has no CPU path)");
+    if (t.scalar_type() != at::kFloat) throw std::runtime_error(std::string(name) + " must be float32");
+    return t.contiguous();
+}
+Tensor cuda_any(const Tensor& t, const char* name)
+{
+    if (!t.defined() || !t.is_cuda())
+        throw std::runtime_error(std::string(name) + " must be a CUDA tensor (this rasterizer has no CPU path)");
+    return t.contiguous();
+}
+float* f32(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
+int32_t* i32(const Tensor& t) { return static_cast<int32_t*>(t.data_ptr()); }
+void* stream() { return at::cuda::getCurrentCUDAStream().stream(); }
+
+Tensor empty_f32(at::IntArrayRef shape, const Tensor& like) { return at::empty(shape, like.options().dtype(at::kFloat).requires_grad(false)); }
+Tensor empty_i32(at::IntArrayRef shape, const Tensor& like) { return at::empty(shape, like.options().dtype(at::kInt).requires_grad(false)); }
+
+// The fields of GaussianRasterizationSettings, by position.
+struct Settings {
+    int H, W;
+    float tanfovx, tanfovy, scale_modifier;
+    Tensor bg, view, proj, campos;
+    bool geo;
+};
+Tensor tensor_item(PyObject* tuple, int i) { return py::handle(PyTuple_GET_ITEM(tuple, i)).cast<Tensor>(); }
+Settings read_settings(const py::handle& h)
+{
+    PyObject* t = h.ptr();
+    if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) != 13) throw std::runtime_error("raster_settings must be a GaussianRasterizationSettings");
+    auto num = [&](int i) { return py::handle(PyTuple_GET_ITEM(t, i)); };
+    Settings s;
+    s.H = num(0).cast<int>();
+    s.W = num(1).cast<int>();
+    s.tanfovx = (float)num(2).cast<double>();
+    s.tanfovy = (float)num(3).cast<double>();
+    s.bg = tensor_item(t, 4);
+    s.scale_modifier = (float)num(5).cast<double>();
+    s.view = tensor_item(t, 6);
+    s.proj = tensor_item(t, 7);
+    s.campos = tensor_item(t, 9);
+    s.geo = PyObject_IsTrue(PyTuple_GET_ITEM(t, 11));
+    return s;
+}
+
+// What a node keeps that is no tensor of the graph.
+template <class T>
+struct Holder : torch::CustomClassHolder {
+    T v;
+    explicit Holder(T x) : v(std::move(x)) {}
+};
+template <class T>
+void keep(AutogradContext* ctx, T v)
+{
+    ctx->saved_data["s"] = c10::IValue::make_capsule(c10::make_intrusive<Holder<T>>(std::move(v)));
+}
+template <class T>
+T& kept(AutogradContext* ctx)
+{
+    return static_cast<Holder<T>*>(ctx->saved_data["s"].toCapsule().get())->v;
+}
+
+// Sub-arrays of one buffer on 128-byte boundaries, in the order in which they are asked for.
+struct Carver {
+    size_t size = 0;
+    size_t add(size_t bytes)
+    {
+        const size_t at = (size + 127) / 128 * 128;
+        size = at + bytes;
+        return at;
+    }
+};
+struct GeometryLayout {
+    size_t tiles_touched, scan, scan_bytes, offsets, num_rendered, records, total;
+    explicit GeometryLayout(int64_t P)
+    {
+        Carver c;
+        tiles_touched = c.add(4 * P);
+        scan_bytes = L.cgx_bin_workspace_bytes((int)P);
+        scan = c.add(scan_bytes);
+        offsets = c.add(4 * P);
+        num_rendered = c.add(4 * 32);
+        records = c.add(L.cgx_render_records_bytes((int)P));
+        total = c.size + 128;
+    }
+};
+struct BinningLayout {
+    size_t list, list_unsorted, keys, keys_unsorted, sort, sort_bytes, total;
+    explicit BinningLayout(int64_t R)
+    {
+        Carver c;
+        list = c.add(4 * R);
+        list_unsorted = c.add(4 * R);
+        keys = c.add(8 * R);
+        keys_unsorted = c.add(8 * R);
+        sort_bytes = L.cgx_sort_workspace_bytes(R);
+        sort = c.add(sort_bytes);
+        total = c.size + 128;
+    }
+};
+struct ImageLayout {
+    size_t accum_alpha, n_contrib, n_contrib2loss, ranges, total;
+    ImageLayout(int64_t N, int64_t T)
+    {
+        Carver c;
+        accum_alpha = c.add(4 * N);
+        n_contrib = c.add(4 * N);
+        n_contrib2loss = c.add(4 * N);
+        ranges = c.add(8 * T);
+        total = c.size + 128;
+    }
+};
+Tensor bytes_like(size_t n, const Tensor& like) { return at::empty({(int64_t)n}, like.options().dtype(at::kByte).requires_grad(false)); }
+template <class T>
+T* at_offset(const Tensor& buf, size_t off)
+{
+    return reinterpret_cast<T*>(static_cast<char*>(buf.data_ptr()) + off);
+}
+
+// ---------------------------------------------------------------------------------------------- elapsed milliseconds
+// Resolved on first numeric use, so that the operators never block the host.
+struct EventMs {
+    cudaEvent_t a = nullptr, b = nullptr;
+    double ms = 0;
+    bool have = false;
+    EventMs()
+    {
+        cudaEventCreate(&a);
+        cudaEventCreate(&b);
+    }
+    EventMs(const EventMs&) = delete;
+    ~EventMs()
+    {
+        if (a) cudaEventDestroy(a);
+        if (b) cudaEventDestroy(b);
+    }
+    double get()
+    {
+        if (!have) {
+            float f = 0.f;
+            cudaEventSynchronize(b);
+            cudaEventElapsedTime(&f, a, b);
+            ms = f;
+            have = true;
+        }
+        return ms;
+    }
+};
+
+// The caller's stats_collector dict (or nothing), usable without the interpreter lock.
+using Stats = std::shared_ptr<PyObject>;
+Stats hold(const py::object& o)
+{
+    if (o.is_none()) return nullptr;
+    return Stats(o.inc_ref().ptr(), [](PyObject* p) {
+        if (!Py_IsInitialized()) return;
+        py::gil_scoped_acquire gil;
+        Py_DECREF(p);
+    });
+}
+void report(const Stats& stats, const char* key, std::shared_ptr<EventMs> ms)
+{
+    py::gil_scoped_acquire gil;
+    py::object v = py::cast(std::move(ms));
+    if (PyObject_SetItem(stats.get(), py::str(key).ptr(), v.ptr()) != 0) throw py::error_already_set();
+}
+
+// ---------------------------------------------------------------------------------------------- pair counts
+// The counting stage leaves (pairs, smallest and largest depth word) in page-locked memory, with a flag behind them that
+// the host watches: neither a copy nor an event stands between the kernel and the launches that need the count.
+constexpr int SLOTS = 256;
+struct Slot {
+    volatile uint32_t pairs, dmin, dmax, flag;
+};
+Slot* slots()
+{
+    static Slot* mem = [] {
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, SLOTS * sizeof(Slot), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
+            throw std::runtime_error("no page-locked memory for the pair counts");
+        return static_cast<Slot*>(p);
+    }();
+    return mem;
+}
+struct Count {
+    Tensor geom;
+    int slot = -1;
+    cudaStream_t stream = nullptr;
+    bool ranged = false;
+    Tensor keep[3];            // a prefetched count's inputs: their addresses stay taken
+};
+std::mutex slot_lock;
+std::vector<int> free_slots = [] {
+    std::vector<int> v;
+    for (int i = SLOTS - 1; i >= 0; i--) v.push_back(i);
+    return v;
+}();
+int take_slot()
+{
+    std::lock_guard<std::mutex> g(slot_lock);
+    if (free_slots.empty()) throw std::runtime_error("too many pair counts in flight");
+    const int s = free_slots.back();
+    free_slots.pop_back();
+    return s;
+}
+void give_slot(int s)
+{
+    std::lock_guard<std::mutex> g(slot_lock);
+    free_slots.push_back(s);
+}
+
+Count start_count(int64_t P, int W, int H, const Tensor& means2D, const Tensor& radii, const Tensor& depths,
+                  const Tensor& local)
+{
+    const GeometryLayout gl(P);
+    Count c;
+    c.geom = bytes_like(gl.total, means2D);
+    c.slot = take_slot();
+    c.stream = at::cuda::getCurrentCUDAStream().stream();
+    c.ranged = depths.defined();
+    Slot& s = slots()[c.slot];
+    s.flag = 0;
+    check(L.cgx_bin_count_scan_post((int)P, W, H, i32(radii), f32(means2D), f32(depths),
+                                    static_cast<uint8_t*>(local.data_ptr()), at_offset<uint32_t>(c.geom, gl.tiles_touched),
+                                    at_offset<uint32_t>(c.geom, gl.num_rendered), at_offset<void>(c.geom, gl.scan),
+                                    gl.scan_bytes, const_cast<uint32_t*>(&s.pairs), c.stream),
+          "cgx_bin_count_scan");
+    return c;
+}
+// Waits for the count; gives the slot back.
+void finish_count(Count& c, int64_t& R, int& low_bits)
+{
+    Slot& s = slots()[c.slot];
+    const auto t0 = std::chrono::steady_clock::now();
+    int spins = 0;
+    while (!s.flag) {
+        if (++spins % 1024 == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(2)) {
+            // a long queue in front of it, or an error: let the driver wait, and say so if there was one
+            const cudaError_t e = cudaStreamSynchronize(c.stream);
+            if (e != cudaSuccess) throw std::runtime_error(std::string("cgx_bin_count_scan: ") + cudaGetErrorString(e));
+            if (!s.flag) throw std::runtime_error("cgx_bin_count_scan: the pair count did not arrive");
+        }
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    R = s.pairs;
+    const uint32_t lo = s.dmin, hi = s.dmax;
+    low_bits = 32;
+    if (c.ranged && lo <= hi) low_bits = lo == hi ? 1 : 32 - __builtin_clz(lo ^ hi);
+    give_slot(c.slot);
+    c.slot = -1;
+}
+
+// Counts started ahead of their render call, found by the identity (and version) of its inputs.
+using PrefetchKey = std::array<int64_t, 10>;
+PrefetchKey prefetch_key(const Tensor& m, const Tensor& r, const Tensor& l, int H, int W)
+{
+    return {(int64_t)m.data_ptr(), (int64_t)r.data_ptr(), (int64_t)l.data_ptr(), m.size(0), H, W, m.device().index(),
+            (int64_t)m._version(), (int64_t)r._version(), (int64_t)l._version()};
+}
+std::mutex prefetch_lock;
+std::map<PrefetchKey, Count> prefetched;
+constexpr size_t PREFETCH_MOST = SLOTS / 2;
+
+bool find_prefetched(Count& c, const Tensor& means2D, const Tensor& radii, const Tensor& local, int H, int W)
+{
+    std::lock_guard<std::mutex> g(prefetch_lock);
+    if (prefetched.empty()) return false;
+    const auto it = prefetched.find(prefetch_key(means2D, radii, local, H, W));
+    if (it == prefetched.end()) return false;
+    c = std::move(it->second);
+    prefetched.erase(it);
+    return true;
+}
+
+void prefetch(int H, int W, const Tensor& means2D_, const Tensor& radii_, const Tensor& local_,
+              const c10::optional<Tensor>& depths_)
+{
+    const Tensor means2D = cuda_f32(means2D_, "means2D"), radii = cuda_any(radii_, "radii"),
+                 local = cuda_any(local_, "compute_locally");
+    const int64_t P = means2D.size(0);
+    if (P == 0 || radii.scalar_type() != at::kInt) return;
+    const c10::cuda::CUDAGuard guard(means2D.device());
+    std::lock_guard<std::mutex> g(prefetch_lock);
+    if (prefetched.size() >= PREFETCH_MOST) {              // counts nobody picked up
+        for (auto& e : prefetched) {
+            int64_t R;
+            int bits;
+            finish_count(e.second, R, bits);
+        }
+        prefetched.clear();
+    }
+    const PrefetchKey key = prefetch_key(means2D, radii, local, H, W);
+    const auto old = prefetched.find(key);
+    if (old != prefetched.end()) {
+        int64_t R;
+        int bits;
+        finish_count(old->second, R, bits);
+        prefetched.erase(old);
+    }
+    Count c = start_count(P, W, H, means2D, radii, depths_ ? cuda_f32(*depths_, "depths") : Tensor(), local);
+    c.keep[0] = means2D;
+    c.keep[1] = radii;
+    c.keep[2] = local;
+    prefetched.emplace(key, std::move(c));
+}
+
+// (geometry buffer, pairs, varying depth bits) of a count started ahead, or None.
+py::object take_prefetched(int H, int W, const Tensor& means2D, const Tensor& radii, const Tensor& local)
+{
+    Count c;
+    int64_t R = 0;
+    int bits = 32;
+    {
+        py::gil_scoped_release nogil;
+        if (!find_prefetched(c, means2D, radii, local, H, W)) c.slot = -1;
+        else finish_count(c, R, bits);
+    }
+    if (!c.geom.defined()) return py::none();
+    return py::make_tuple(c.geom, R, bits);
+}
+size_t prefetched_counts()
+{
+    std::lock_guard<std::mutex> g(prefetch_lock);
+    return prefetched.size();
+}
+
+// ---------------------------------------------------------------------------------------------- render
+struct RenderState {
+    int64_t P, R;
+    int H, W;
+    float tanfovx, tanfovy;
+    bool geo;
+    Stats stats;
+};
+
+struct Render : torch::autograd::Function<Render> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& means2D_, const c10::optional<Tensor>& means2D_abs,
+                                 const Tensor& conic_, const Tensor& rgb_, const Tensor& all_map_, const Tensor& depths_,
+                                 const Tensor& radii_, const Tensor& local_, const Tensor& local_bwd, const Settings& s,
+                                 const Stats& stats)
+    {
+        const Tensor means2D = cuda_f32(means2D_, "means2D");
+        const int64_t P = means2D.size(0);
+        const int H = s.H, W = s.W;
+        const int64_t T = (int64_t)((W + 15) / 16) * ((H + 15) / 16), HW = (int64_t)H * W;
+        const Tensor depths = cuda_f32(depths_, "depths"), conic = cuda_f32(conic_, "conic_opacity"),
+                     rgb = cuda_f32(rgb_, "rgb"), all_map = cuda_f32(all_map_, "all_map"),
+                     radii = cuda_any(radii_, "radii").to(at::kInt), local = cuda_any(local_, "compute_locally"),
+                     bg = cuda_f32(s.bg, "background");
+        if (local.scalar_type() != at::kBool || local.numel() != T)
+            throw std::runtime_error("compute_locally must be a bool tensor with one entry per tile");
+        if (means2D.size(1) != 2 || conic.numel() != 4 * P || rgb.numel() != 3 * P || all_map.numel() != 5 * P ||
+            conic.size(0) != P || rgb.size(0) != P || all_map.size(0) != P || depths.numel() != P || radii.numel() != P)
+            throw std::runtime_error("render_gaussians: per-Gaussian tensors must be (P,2) (P,4) (P,3) (P,5) (P) (P)");
+        const c10::cuda::CUDAGuard guard(means2D.device());
+        const cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
+
+        Count count;
+        if (!find_prefetched(count, means2D, radii, local, H, W))
+            count = start_count(P, W, H, means2D, radii, depths, local);
+        // allocated while the count is on its way
+        const GeometryLayout gl(P);
+        const ImageLayout il(HW, T);
+        const Tensor n_render = empty_i32({T}, means2D), n_consider = empty_i32({T}, means2D),
+                     n_contrib = empty_i32({T}, means2D), observe = empty_i32({P}, means2D),
+                     color = empty_f32({3, H, W}, means2D), out_map = empty_f32({5, H, W}, means2D),
+                     depth = empty_f32({1, H, W}, means2D), img = bytes_like(il.total, means2D);
+        std::shared_ptr<EventMs> ms = stats ? std::make_shared<EventMs>() : nullptr;
+        const int bit = (int)L.cgx_higher_msb((uint32_t)T);
+        int64_t R;
+        int low_bits;
+        finish_count(count, R, low_bits);
+
+        const BinningLayout bl(R);
+        const Tensor bin = bytes_like(bl.total, means2D);
+        if (ms) cudaEventRecord(ms->a, st);
+        // the sort ping-pongs between the two key/value arrays: the pairs are emitted into whichever array makes the last
+        // pass land in keys / list
+        const bool even = L.cgx_sort_passes(low_bits + bit) % 2 == 0;
+        uint64_t* keys[2] = {at_offset<uint64_t>(bin, bl.keys), at_offset<uint64_t>(bin, bl.keys_unsorted)};
+        uint32_t* list[2] = {at_offset<uint32_t>(bin, bl.list), at_offset<uint32_t>(bin, bl.list_unsorted)};
+        const int first = even ? 0 : 1;
+        uint32_t* tiles = at_offset<uint32_t>(count.geom, gl.tiles_touched);
+        uint8_t* loc = static_cast<uint8_t*>(local.data_ptr());
+        uint32_t* ranges = at_offset<uint32_t>(img, il.ranges);
+        check(L.cgx_emit_keys((int)P, W, H, i32(radii), f32(means2D), f32(depths), tiles, loc,
+                              at_offset<uint32_t>(count.geom, gl.offsets), keys[first], list[first], R,
+                              at_offset<void>(count.geom, gl.scan), st), "cgx_emit_keys");
+        check(L.cgx_sort_pairs_pingpong(R, 32 + bit, low_bits, keys[first], list[first], keys[1 - first], list[1 - first],
+                                        at_offset<void>(bin, bl.sort), bl.sort_bytes, 0, st), "cgx_sort_pairs");
+        check(L.cgx_tile_ranges(R, (int)T, keys[0], ranges, st), "cgx_tile_ranges");
+        check(L.cgx_render_fwd((int)P, W, H, s.tanfovx, s.tanfovy, ranges, list[0], i32(radii), f32(means2D), f32(rgb),
+                               f32(all_map), f32(conic), loc, f32(bg), s.geo, at_offset<void>(count.geom, gl.records),
+                               at_offset<float>(img, il.accum_alpha), at_offset<uint32_t>(img, il.n_contrib),
+                               at_offset<uint32_t>(img, il.n_contrib2loss), f32(color), i32(observe), f32(out_map),
+                               f32(depth), i32(n_render), i32(n_consider), i32(n_contrib), st), "cgx_render_fwd");
+        if (ms) {
+            cudaEventRecord(ms->b, st);
+            report(stats, "forward_render_time", std::move(ms));
+        }
+        ctx->set_materialize_grads(false);
+        ctx->mark_non_differentiable({n_render, n_consider, n_contrib, observe});
+        ctx->save_for_backward({out_map, count.geom, bin, img, cuda_any(local_bwd, "compute_locally"), bg});
+        keep(ctx, RenderState{P, R, H, W, s.tanfovx, s.tanfovy, s.geo, stats});
+        return {color, n_render, n_consider, n_contrib, observe, out_map, depth};
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list g)
+    {
+        const RenderState& s = kept<RenderState>(ctx);
+        const variable_list saved = ctx->get_saved_variables();
+        const Tensor &out_map = saved[0], &geom = saved[1], &bin = saved[2], &img = saved[3], &local = saved[4], &bg = saved[5];
+        const c10::cuda::CUDAGuard guard(out_map.device());
+        const cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
+        auto cotangent = [&](const Tensor& t, int n, const char* name, bool needed) {
+            if (t.defined()) return cuda_f32(t, name);
+            return needed ? at::zeros({n, s.H, s.W}, out_map.options()) : Tensor();
+        };
+        const Tensor d_color = cotangent(g[0], 3, "dL_dout_color", true), d_map = cotangent(g[5], 5, "dL_dout_all_map", s.geo),
+                     d_depth = cotangent(g[6], 1, "dL_dout_plane_depth", s.geo);
+        const int64_t P = s.P, HW = (int64_t)s.H * s.W, T = (int64_t)((s.W + 15) / 16) * ((s.H + 15) / 16);
+        const GeometryLayout gl(P);
+        const BinningLayout bl(s.R);
+        const ImageLayout il(HW, T);
+        const Tensor m2 = empty_f32({P, 2}, out_map), abs2 = empty_f32({P, 3}, out_map), co = empty_f32({P, 4}, out_map),
+                     rgb = empty_f32({P, 3}, out_map), am = empty_f32({P, 5}, out_map);
+        const size_t ws_bytes = L.cgx_render_bwd_workspace_bytes((int)P);
+        const Tensor ws = bytes_like(ws_bytes, out_map);
+        std::shared_ptr<EventMs> ms = s.stats ? std::make_shared<EventMs>() : nullptr;
+        if (ms) cudaEventRecord(ms->a, st);
+        check(L.cgx_render_bwd_table((int)P, s.W, s.H, s.tanfovx, s.tanfovy, at_offset<uint32_t>(img, il.ranges),
+                                     at_offset<uint32_t>(bin, bl.list), f32(bg), at_offset<void>(geom, gl.records),
+                                     f32(out_map), at_offset<float>(img, il.accum_alpha),
+                                     at_offset<uint32_t>(img, il.n_contrib), static_cast<uint8_t*>(local.data_ptr()),
+                                     f32(d_color), f32(d_map), f32(d_depth), s.geo, f32(m2), f32(abs2), f32(co), f32(rgb),
+                                     f32(am), 0, at_offset<uint32_t>(geom, gl.tiles_touched), ws.data_ptr(), ws_bytes, st),
+              "cgx_render_bwd");
+        if (ms) {
+            cudaEventRecord(ms->b, st);
+            report(s.stats, "backward_render_time", std::move(ms));
+        }
+        return {m2, abs2, co, rgb, am, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+
+std::vector<Tensor> render(const Tensor& means2D, const c10::optional<Tensor>& means2D_abs, const Tensor& conic,
+                           const Tensor& rgb, const Tensor& all_map, const Tensor& depths, const Tensor& radii,
+                           const Tensor& local, const Tensor& local_bwd, const py::object& settings, const py::object& stats)
+{
+    const Settings s = read_settings(settings);
+    const Stats held = hold(stats);
+    py::gil_scoped_release nogil;
+    return Render::apply(means2D, means2D_abs, conic, rgb, all_map, depths, radii, local, local_bwd, s, held);
+}
+
+// ---------------------------------------------------------------------------------------------- preprocess
+struct Preprocess : torch::autograd::Function<Preprocess> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& means3D_, const Tensor& scales_,
+                                 const Tensor& rotations_, const Tensor& sh, const Tensor& opacities_, const Settings& s)
+    {
+        if (means3D_.dim() != 2 || means3D_.size(1) != 3)
+            throw std::runtime_error("means3D must have dimensions (num_points, 3)");
+        const Tensor means3D = cuda_f32(means3D_, "means3D");
+        const int64_t P = means3D.size(0);
+        const c10::cuda::CUDAGuard guard(means3D.device());
+        const Tensor m2 = empty_f32({P, 2}, means3D), depths = empty_f32({P}, means3D), radii = empty_i32({P}, means3D),
+                     co = empty_f32({P, 4}, means3D);
+        // SH evaluation is compiled out upstream: rgb stays zero
+        const Tensor rgb = at::zeros({P, 3}, means3D.options().requires_grad(false));
+        const Tensor scales = cuda_f32(scales_, "scales"), rotations = cuda_f32(rotations_, "rotations"),
+                     opacities = cuda_f32(opacities_, "opacity"), view = cuda_f32(s.view, "viewmatrix"),
+                     proj = cuda_f32(s.proj, "projmatrix");
+        if (P)
+            check(L.cgx_preprocess_fwd((int)P, f32(means3D), f32(scales), s.scale_modifier, f32(rotations), f32(opacities),
+                                       f32(view), f32(proj), s.W, s.H, s.tanfovx, s.tanfovy, f32(m2), f32(depths),
+                                       i32(radii), nullptr, f32(co), stream()), "cgx_preprocess_fwd");
+        ctx->set_materialize_grads(false);
+        ctx->mark_non_differentiable({radii, depths});
+        ctx->save_for_backward({means3D_, scales_, rotations_, radii, view, proj});
+        Settings lean = s;
+        lean.bg = lean.view = lean.proj = lean.campos = Tensor();
+        keep(ctx, std::make_pair(lean, sh.requires_grad()));
+        return {m2, rgb, co, radii, depths};
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g)
+    {
+        const auto& k = kept<std::pair<Settings, bool>>(ctx);
+        const Settings& s = k.first;
+        const variable_list v = ctx->get_saved_variables();
+        const Tensor means3D = v[0].contiguous(), scales = v[1].contiguous(), rotations = v[2].contiguous();
+        const int64_t P = means3D.size(0);
+        const c10::cuda::CUDAGuard guard(means3D.device());
+        const auto opt = means3D.options().requires_grad(false);
+        const Tensor g_m2 = g[0].defined() ? cuda_f32(g[0], "dL_dmeans2D") : at::zeros({P, 2}, opt);
+        const Tensor g_co = g[2].defined() ? cuda_f32(g[2], "dL_dconic_opacity") : at::zeros({P, 4}, opt);
+        const Tensor dm = empty_f32({P, 3}, means3D), ds = empty_f32({P, 3}, means3D), dr = empty_f32({P, 4}, means3D),
+                     dop = empty_f32({P, 1}, means3D);
+        if (P)
+            check(L.cgx_preprocess_bwd((int)P, f32(means3D), f32(scales), s.scale_modifier, f32(rotations), i32(v[3]),
+                                       f32(v[4]), f32(v[5]), s.W, s.H, s.tanfovx, s.tanfovy, f32(g_m2), f32(g_co), f32(dm),
+                                       f32(ds), f32(dr), f32(dop), stream()), "cgx_preprocess_bwd");
+        return {dm, ds, dr, k.second ? at::zeros({P, 3}, opt) : Tensor(), dop, Tensor()};
+    }
+};
+
+std::vector<Tensor> preprocess(const Tensor& means3D, const Tensor& scales, const Tensor& rotations, const Tensor& sh,
+                               const Tensor& opacities, const py::object& settings)
+{
+    const Settings s = read_settings(settings);
+    py::gil_scoped_release nogil;
+    return Preprocess::apply(means3D, scales, rotations, sh, opacities, s);
+}
+
+// All cameras of a batch in one launch; per camera means2D, conic_opacity, radii, depths[, all_map].
+struct Cameras {
+    std::vector<cgx_camera> cam;
+    std::vector<Tensor> matrices, campos;
+    float scale_modifier = 1.f;
+    bool planes = false;
+};
+constexpr size_t MAX_CAMS = 16;
+
+struct PreprocessBatch : torch::autograd::Function<PreprocessBatch> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& means3D_, const Tensor& scales_,
+                                 const Tensor& rotations_, const Tensor& opacities_, std::shared_ptr<Cameras> c)
+    {
+        if (means3D_.dim() != 2 || means3D_.size(1) != 3)
+            throw std::runtime_error("means3D must have dimensions (num_points, 3)");
+        const Tensor means3D = cuda_f32(means3D_, "means3D"), scales = cuda_f32(scales_, "scales"),
+                     rotations = cuda_f32(rotations_, "rotations"), opacities = cuda_f32(opacities_, "opacities");
+        const int64_t P = means3D.size(0);
+        const size_t B = c->cam.size();
+        const c10::cuda::CUDAGuard guard(means3D.device());
+        variable_list out, fixed, saved = {means3D_, scales_, rotations_};
+        float *m2[MAX_CAMS], *dep[MAX_CAMS], *co[MAX_CAMS], *am[MAX_CAMS];
+        int32_t* rad[MAX_CAMS];
+        const float* campos[MAX_CAMS];
+        for (size_t b = 0; b < B; b++) {
+            const Tensor t_m2 = empty_f32({P, 2}, means3D), t_co = empty_f32({P, 4}, means3D),
+                         t_rad = empty_i32({P}, means3D), t_dep = empty_f32({P}, means3D);
+            m2[b] = f32(t_m2), co[b] = f32(t_co), rad[b] = i32(t_rad), dep[b] = f32(t_dep);
+            out.insert(out.end(), {t_m2, t_co, t_rad, t_dep});
+            if (c->planes) {
+                const Tensor t_am = empty_f32({P, 5}, means3D);
+                am[b] = f32(t_am);
+                campos[b] = f32(c->campos[b]);
+                out.push_back(t_am);
+            }
+            fixed.insert(fixed.end(), {t_rad, t_dep});
+            saved.push_back(t_rad);
+        }
+        if (P)
+            check(L.cgx_preprocess_fwd_batched_planes((int)P, (int)B, f32(means3D), f32(scales), c->scale_modifier,
+                                                      f32(rotations), f32(opacities), c->cam.data(),
+                                                      c->planes ? campos : nullptr, m2, dep, rad, co,
+                                                      c->planes ? am : nullptr, stream()), "cgx_preprocess_fwd_batched");
+        ctx->set_materialize_grads(false);
+        ctx->mark_non_differentiable(fixed);
+        ctx->save_for_backward(std::move(saved));
+        keep(ctx, std::move(c));
+        return out;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g)
+    {
+        const Cameras& c = *kept<std::shared_ptr<Cameras>>(ctx);
+        const variable_list v = ctx->get_saved_variables();
+        const Tensor means3D = v[0].contiguous(), scales = v[1].contiguous(), rotations = v[2].contiguous();
+        const int64_t P = means3D.size(0);
+        const size_t B = c.cam.size(), n_out = c.planes ? 5 : 4;
+        const c10::cuda::CUDAGuard guard(means3D.device());
+        const auto opt = means3D.options().requires_grad(false);
+        const Tensor dm = empty_f32({P, 3}, means3D), ds = empty_f32({P, 3}, means3D), dr = empty_f32({P, 4}, means3D),
+                     dop = empty_f32({P, 1}, means3D);
+        std::vector<cgx_camera> cam;
+        std::vector<Tensor> hold;
+        const float *gm[MAX_CAMS], *gc[MAX_CAMS], *ga[MAX_CAMS], *campos[MAX_CAMS];
+        const int32_t* rad[MAX_CAMS];
+        bool planes = false;
+        auto ready = [&](const Tensor& t, int64_t n) {
+            hold.push_back(t.defined() ? cuda_f32(t, "cotangent") : at::zeros({P, n}, opt));
+            return (const float*)f32(hold.back());
+        };
+        for (size_t b = 0; b < B; b++) {
+            const Tensor &m = g[n_out * b], &o = g[n_out * b + 1];
+            const Tensor a = c.planes ? g[n_out * b + 4] : Tensor();
+            if (!m.defined() && !o.defined() && !a.defined()) continue;      // no cotangent: contributes nothing
+            const size_t i = cam.size();
+            cam.push_back(c.cam[b]);
+            gm[i] = ready(m, 2);
+            gc[i] = ready(o, 4);
+            ga[i] = a.defined() ? ready(a, 5) : nullptr;
+            planes |= a.defined();
+            campos[i] = c.planes ? f32(c.campos[b]) : nullptr;
+            rad[i] = i32(v[3 + b]);
+        }
+        if (P && !cam.empty()) {
+            check(L.cgx_preprocess_bwd_batched_planes((int)P, (int)cam.size(), f32(means3D), f32(scales), c.scale_modifier,
+                                                      f32(rotations), cam.data(), planes ? campos : nullptr, rad, gm, gc,
+                                                      planes ? ga : nullptr, f32(dm), f32(ds), f32(dr), f32(dop), stream()),
+                  "cgx_preprocess_bwd_batched");
+        } else {
+            for (const Tensor& t : {dm, ds, dr, dop}) t.zero_();
+        }
+        return {dm, ds, dr, dop, Tensor()};
+    }
+};
+
+std::vector<Tensor> preprocess_batched(const Tensor& means3D, const Tensor& scales, const Tensor& rotations,
+                                       const Tensor& opacities, const py::list& settings, bool planes)
+{
+    const size_t B = settings.size();
+    if (!means3D.is_cuda()) throw std::runtime_error("means3D must be a CUDA tensor (this rasterizer has no CPU path)");
+    if (B < 1 || B > MAX_CAMS) throw std::runtime_error("between 1 and 16 cameras per batched call");
+    auto c = std::make_shared<Cameras>();
+    c->planes = planes;
+    for (size_t b = 0; b < B; b++) {
+        const Settings s = read_settings(settings[b]);
+        if (b == 0) c->scale_modifier = s.scale_modifier;
+        if (!s.view.is_cuda() || !s.proj.is_cuda()) throw std::runtime_error("camera matrices must be CUDA tensors");
+        const Tensor view = s.view.contiguous(), proj = s.proj.contiguous();
+        c->matrices.insert(c->matrices.end(), {view, proj});
+        if (planes) c->campos.push_back(s.campos.contiguous());
+        cgx_camera k;
+        k.viewmatrix = f32(view);
+        k.projmatrix = f32(proj);
+        k.tanfovx = s.tanfovx;
+        k.tanfovy = s.tanfovy;
+        k.W = s.W;
+        k.H = s.H;
+        c->cam.push_back(k);
+    }
+    py::gil_scoped_release nogil;
+    return PreprocessBatch::apply(means3D, scales, rotations, opacities, c);
+}
+
+// ---------------------------------------------------------------------------------------------- plane descriptors
+struct PlaneMap : torch::autograd::Function<PlaneMap> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& means3D_, const Tensor& scales_, const Tensor& rotations_,
+                          const c10::optional<Tensor>& radii_, const Tensor& view_, const Tensor& campos_)
+    {
+        auto ready = [](const Tensor& t, const char* name) {
+            if (!t.is_cuda() || t.scalar_type() != at::kFloat)
+                throw std::runtime_error(std::string("plane_map: ") + name + " must be a float32 CUDA tensor (no CPU path)");
+            return t.contiguous();
+        };
+        const Tensor means3D = ready(means3D_, "means3D"), scales = ready(scales_, "scales"),
+                     rotations = ready(rotations_, "rotations"), view = ready(view_, "viewmatrix"),
+                     campos = ready(campos_, "campos");
+        const Tensor radii = radii_ && radii_->defined() ? radii_->contiguous() : Tensor();
+        const int64_t P = means3D.size(0);
+        const c10::cuda::CUDAGuard guard(means3D.device());
+        const Tensor out = empty_f32({P, 5}, means3D);
+        if (P)
+            check(L.cgx_all_map_fwd((int)P, f32(means3D), f32(scales), f32(rotations), radii.defined() ? i32(radii) : nullptr,
+                                    f32(view), f32(campos), f32(out), stream()), "cgx_all_map_fwd");
+        ctx->save_for_backward({means3D, scales, rotations, radii, view, campos});
+        return out;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g)
+    {
+        const variable_list v = ctx->get_saved_variables();
+        const Tensor &means3D = v[0], &radii = v[3], g5 = g[0].contiguous();
+        const int64_t P = means3D.size(0);
+        const c10::cuda::CUDAGuard guard(means3D.device());
+        const Tensor dm = empty_f32({P, 3}, means3D), dr = empty_f32({P, 4}, means3D);
+        if (P)
+            check(L.cgx_all_map_bwd((int)P, f32(means3D), f32(v[1]), f32(v[2]), radii.defined() ? i32(radii) : nullptr,
+                                    f32(v[4]), f32(v[5]), f32(g5), f32(dm), f32(dr), stream()), "cgx_all_map_bwd");
+        return {dm, Tensor(), dr, Tensor(), Tensor(), Tensor()};
+    }
+};
+Tensor plane_map(const Tensor& means3D, const Tensor& scales, const Tensor& rotations, const c10::optional<Tensor>& radii,
+                 const Tensor& view, const Tensor& campos)
+{
+    return PlaneMap::apply(means3D, scales, rotations, radii, view, campos);
+}
+
+// ---------------------------------------------------------------------------------------------- loss
+struct StripLoss : torch::autograd::Function<StripLoss> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& image_, const Tensor& gt_,
+                                 const c10::optional<Tensor>& mask_)
+    {
+        if (!image_.is_cuda() || image_.scalar_type() != at::kFloat || !gt_.is_cuda() || gt_.scalar_type() != at::kFloat)
+            throw std::runtime_error("strip_loss: image and gt must be float32 CUDA tensors (no CPU path)");
+        if (image_.dim() != 3 || gt_.sizes() != image_.sizes())
+            throw std::runtime_error("strip_loss: image and gt must both be (C, H, W)");
+        const Tensor image = image_.contiguous(), gt = gt_.contiguous();
+        const int64_t C = image.size(0), H = image.size(1), W = image.size(2);
+        Tensor mask;
+        if (mask_ && mask_->defined()) {
+            if (mask_->dim() != 2 || mask_->size(0) != H || mask_->size(1) != W || !mask_->is_cuda())
+                throw std::runtime_error("strip_loss: mask must be a (H, W) CUDA tensor");
+            mask = mask_->to(at::kBool).contiguous();
+        }
+        const c10::cuda::CUDAGuard guard(image.device());
+        const Tensor sums = at::empty({2}, image.options().dtype(at::kDouble).requires_grad(false));
+        // the three derivative maps are for the backward pass
+        const Tensor maps = image_.requires_grad() ? empty_f32({3, C, H, W}, image) : Tensor();
+        const int64_t n = C * H * W;
+        float* m = f32(maps);
+        if (n)
+            check(L.cgx_strip_loss_fwd((int)C, (int)H, (int)W, f32(image), f32(gt),
+                                       mask.defined() ? static_cast<uint8_t*>(mask.data_ptr()) : nullptr,
+                                       static_cast<double*>(sums.data_ptr()), m, m ? m + n : nullptr,
+                                       m ? m + 2 * n : nullptr, stream()), "cgx_strip_loss_fwd");
+        else
+            sums.zero_();
+        ctx->set_materialize_grads(false);
+        ctx->save_for_backward({image, gt, mask, maps});
+        const Tensor f = sums.to(at::kFloat);
+        return {f.select(0, 0), f.select(0, 1)};
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g)
+    {
+        const variable_list v = ctx->get_saved_variables();
+        const Tensor &image = v[0], &mask = v[2];
+        const int64_t C = image.size(0), H = image.size(1), W = image.size(2), n = C * H * W;
+        const c10::cuda::CUDAGuard guard(image.device());
+        const auto opt = image.options().requires_grad(false);
+        Tensor w[2];
+        for (int k = 0; k < 2; k++) w[k] = g[k].defined() ? g[k].to(at::kFloat) : at::zeros({}, opt);
+        const Tensor weights = at::stack({w[0], w[1]}), grad = at::empty_like(image);
+        const float* m = f32(v[3]);
+        if (n)
+            check(L.cgx_strip_loss_bwd((int)C, (int)H, (int)W, f32(image), f32(v[1]),
+                                       mask.defined() ? static_cast<uint8_t*>(mask.data_ptr()) : nullptr, f32(weights), m,
+                                       m + n, m + 2 * n, f32(grad), stream()), "cgx_strip_loss_bwd");
+        return {grad, Tensor(), Tensor()};
+    }
+};
+std::vector<Tensor> strip_loss(const Tensor& image, const Tensor& gt, const c10::optional<Tensor>& mask)
+{
+    return StripLoss::apply(image, gt, mask);
+}
+
+struct DepthNormal : torch::autograd::Function<DepthNormal> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& depth_, double fx, double fy, double cx, double cy)
+    {
+        if (!depth_.is_cuda() || depth_.scalar_type() != at::kFloat || depth_.dim() != 2)
+            throw std::runtime_error("depth_normal: depth must be a (H, W) float32 CUDA tensor (no CPU path)");
+        const Tensor depth = depth_.contiguous();
+        const int64_t H = depth.size(0), W = depth.size(1);
+        const c10::cuda::CUDAGuard guard(depth.device());
+        const Tensor normal = empty_f32({3, H, W}, depth);
+        if (H * W)
+            check(L.cgx_depth_normal_fwd((int)H, (int)W, (float)fx, (float)fy, (float)cx, (float)cy, f32(depth),
+                                         f32(normal), stream()), "cgx_depth_normal_fwd");
+        ctx->save_for_backward({depth});
+        keep(ctx, std::array<float, 4>{(float)fx, (float)fy, (float)cx, (float)cy});
+        return normal;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g)
+    {
+        const Tensor depth = ctx->get_saved_variables()[0];
+        const auto& k = kept<std::array<float, 4>>(ctx);
+        const c10::cuda::CUDAGuard guard(depth.device());
+        const Tensor out = at::empty_like(depth), gn = g[0].contiguous();
+        if (depth.numel())
+            check(L.cgx_depth_normal_bwd((int)depth.size(0), (int)depth.size(1), k[0], k[1], k[2], k[3], f32(depth), f32(gn),
+                                         f32(out), stream()), "cgx_depth_normal_bwd");
+        return {out, Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+Tensor depth_normal_op(const Tensor& depth, double fx, double fy, double cx, double cy)
+{
+    return DepthNormal::apply(depth, fx, fy, cx, cy);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
+{
+    const auto nogil = py::call_guard<py::gil_scoped_release>();
+    m.def("bind", &bind);
+    m.def("prefetch", &prefetch, nogil);
+    m.def("take_prefetched", &take_prefetched);
+    m.def("prefetched", &prefetched_counts, nogil);
+    m.def("render", &render);
+    m.def("preprocess", &preprocess);
+    m.def("preprocess_batched", &preprocess_batched);
+    m.def("plane_map", &plane_map, nogil);
+    m.def("strip_loss", &strip_loss, nogil);
+    m.def("depth_normal", &depth_normal_op, nogil);
+    auto num = [](const py::object& o) { return py::float_(o).cast<double>(); };
+    py::class_<EventMs, std::shared_ptr<EventMs>>(m, "EventMs")
+        .def("__float__", &EventMs::get)
+        .def("__add__", [num](EventMs& a, const py::object& o) { return a.get() + num(o); })
+        .def("__radd__", [num](EventMs& a, const py::object& o) { return a.get() + num(o); })
+        .def("__mul__", [num](EventMs& a, const py::object& o) { return a.get() * num(o); })
+        .def("__rmul__", [num](EventMs& a, const py::object& o) { return a.get() * num(o); })
+        .def("__sub__", [num](EventMs& a, const py::object& o) { return a.get() - num(o); })
+        .def("__rsub__", [num](EventMs& a, const py::object& o) { return num(o) - a.get(); })
+        .def("__truediv__", [num](EventMs& a, const py::object& o) { return a.get() / num(o); })
+        .def("__repr__", [](EventMs& a) { return std::to_string(a.get()); });
+}

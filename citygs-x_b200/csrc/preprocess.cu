@@ -370,9 +370,12 @@ preprocess_fwd_kernel(int P, const float* __restrict__ means3D, const float* __r
         points_xy_image[idx] = out_xy;
         depths[idx] = out_depth;
         conic_opacity[idx] = out_co;
+        if (cov3Ds) {
 #pragma unroll
-        for (int k = 0; k < 6; k++) s_cov[6 * t + k] = cov3D[k];
+            for (int k = 0; k < 6; k++) s_cov[6 * t + k] = cov3D[k];
+        }
     }
+    if (!cov3Ds) return;          // a quarter of the bytes, for callers that recompute it in the backward pass
     __syncthreads();
     block_store_rows<6>(cov3Ds + (size_t)base * 6, s_cov, count, vec_mask & 8);
 }
@@ -1200,7 +1203,7 @@ static int preprocess_launch(bool filter, int P, const float* means3D, const flo
     if (P == 0) return CGX_OK;
     if (!means3D || !viewmatrix || !projmatrix || !radii) return CGX_EINVAL;
     if (!(filter && cov3D_precomp) && (!scales || !rotations)) return CGX_EINVAL;
-    if (!filter && (!opacities || !means2D || !depths || !cov3D || !conic_opacity)) return CGX_EINVAL;
+    if (!filter && (!opacities || !means2D || !depths || !conic_opacity)) return CGX_EINVAL;
     if (!filter && (((uintptr_t)means2D & 7) || !aligned16(conic_opacity))) return CGX_EINVAL;
     // focal lengths are computed on the host in fp32, as the reference does before launching
     const float focal_y = H / (2.0f * tanfovy);

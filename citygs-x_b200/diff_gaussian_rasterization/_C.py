@@ -257,17 +257,24 @@ def _check_device(dev):
 # synchronisation per call, as in the reference (RAST/cuda_rasterizer/rasterizer_impl.cu:648-660).  A caller that
 # renders several cameras in a row can start the counting stage of ALL of them first (prefetch_num_rendered), so
 # that the first read-back covers every camera and the remaining launches queue back to back with no bubbles.
-# render_gaussians picks a prefetched count up by the identity of its inputs; nothing changes when none exists.
-_PREFETCH = {}
-_PREFETCH_SLOTS = 256
-_prefetch_pinned = None
-_prefetch_next = 0
+# render_gaussians picks a prefetched count up by the identity (and version) of its inputs; nothing changes when none
+# exists.
+class _Prefetched:
+    """The counts that nobody has picked up yet (kept by the C++ host path)."""
+
+    def __len__(self):
+        return _lib.host().prefetched()
 
 
-def _prefetch_key(means2D, radii, local, H, W):
-    # the version counters make a count taken before an in-place update of its inputs unfindable
-    return (means2D.data_ptr(), radii.data_ptr(), local.data_ptr(), means2D.shape[0], H, W, means2D.device.index,
-            means2D._version, radii._version, local._version)
+_PREFETCH = _Prefetched()
+
+
+def prefetch_num_rendered(image_height, image_width, means2D, radii, compute_locally, depths=None):
+    """Launch the tile-count + prefix-sum stage of a coming render_gaussians call with these same tensors and let it
+    post the pair count (and, when `depths` is given, the depth range that lets the sort skip a pass) to pinned host
+    memory without waiting for it.  Not part of the reference's module."""
+    if PROFILE is None:             # under profiling the render call counts for itself, between its own events
+        _lib.host().prefetch(int(image_height), int(image_width), means2D, radii, compute_locally, depths)
 
 
 def _low_bits(dmin, dmax):
@@ -276,41 +283,6 @@ def _low_bits(dmin, dmax):
     if dmin > dmax:
         return 32                      # no pairs
     return max(1, (dmin ^ dmax).bit_length())
-
-
-def prefetch_num_rendered(image_height, image_width, means2D, radii, compute_locally, depths=None):
-    """Launch the tile-count + prefix-sum stage of a coming render_gaussians call with these same tensors and copy
-    the pair count (and, when `depths` is given, the depth range that lets the sort skip a pass) to pinned host
-    memory without waiting for it.  Not part of the reference's module."""
-    global _prefetch_pinned, _prefetch_next
-    l = _lib.lib()
-    means2D = _cuda_f32(means2D, "means2D")
-    radii = _cuda_any(radii, "radii")
-    local = _cuda_any(compute_locally, "compute_locally")
-    P, dev = means2D.shape[0], means2D.device
-    H, W = int(image_height), int(image_width)
-    if P == 0 or radii.dtype != torch.int32:
-        return
-    if _prefetch_pinned is None:
-        _prefetch_pinned = torch.zeros(_PREFETCH_SLOTS, 3, dtype=torch.int32).pin_memory()
-    if len(_PREFETCH) >= _PREFETCH_SLOTS // 2:
-        _PREFETCH.clear()                       # counts nobody picked up
-    slot = _prefetch_next
-    _prefetch_next = (_prefetch_next + 1) % _PREFETCH_SLOTS
-    with torch.cuda.device(dev):
-        glay = geometry_layout(P)
-        geomBuffer = torch.empty(glay.total(), dtype=torch.uint8, device=dev)
-        g = glay.views(geomBuffer)
-        _count_scan(l, P, W, H, radii, means2D, None if depths is None else _cuda_f32(depths, "depths"), local, g,
-                    _stream())
-        # [1:3] only meaningful with depths; a kernel carries the words so they do not wait behind bulk read-backs
-        _lib.check(l.cgx_post_words(_ptr(g["num_rendered"]), C.c_void_p(_prefetch_pinned[slot].data_ptr()), 3,
-                                    _stream()), "cgx_post_words")
-        ev = torch.cuda.Event()
-        ev.record()
-    # the tensors are kept alive with the entry, so their addresses cannot be reused while it exists
-    _PREFETCH[_prefetch_key(means2D, radii, local, H, W)] = (geomBuffer, slot, ev, (means2D, radii, local),
-                                                             depths is not None)
 
 
 def _count_scan(l, P, W, H, radii, means2D, depths, local, g, st):
@@ -368,20 +340,18 @@ def render_gaussians(background, image_height, image_width, means2D, depths, rad
         ilay = image_layout(W * H, T)
         imgBuffer = torch.empty(ilay.total(), dtype=torch.uint8, device=dev)
         im = ilay.views(imgBuffer)
-        pre = _PREFETCH.pop(_prefetch_key(means2D, radii, local, H, W), None) if _PREFETCH else None
+        pre = _lib.host().take_prefetched(H, W, means2D, radii, local)
         if pre is not None:
-            geomBuffer, slot, ev, _, has_range = pre
+            geomBuffer, R, low_bits = pre
             g = glay.views(geomBuffer)
-            ev.synchronize()
-            R, dmin, dmax = _prefetch_pinned[slot].tolist()
-            if not has_range:
-                dmin, dmax = -1, 0
         else:
             geomBuffer = torch.empty(glay.total(), dtype=torch.uint8, device=dev)
             g = glay.views(geomBuffer)
             _count_scan(l, P, W, H, radii, means2D, depths, local, g, st)
             # the key/value buffers are sized from the pair count: one host read, as in the reference
             R, dmin, dmax = g["num_rendered"][0:3].tolist()
+            # depths of one view share their leading bits: the sort squeezes them out of its digits
+            low_bits = _low_bits(dmin, dmax)
 
         blay = binning_layout(R)
         binningBuffer = torch.empty(blay.total(), dtype=torch.uint8, device=dev)
@@ -393,8 +363,6 @@ def render_gaussians(background, image_height, image_width, means2D, depths, rad
         # the sort ping-pongs between the two key/value arrays: the pairs are emitted into whichever array makes
         # the last pass land in point_list_keys / point_list (no copy, whatever the number of passes)
         bit = int(l.cgx_higher_msb(T))
-        # depths of one view share their leading bits: the sort squeezes them out of its digits
-        low_bits = _low_bits(dmin, dmax)
         first = ("point_list_keys", "point_list") if l.cgx_sort_passes(low_bits + bit) % 2 == 0 else \
             ("point_list_keys_unsorted", "point_list_unsorted")
         other = ("point_list_keys_unsorted", "point_list_unsorted") if first[0] == "point_list_keys" else \

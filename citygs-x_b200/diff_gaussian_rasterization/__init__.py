@@ -7,7 +7,9 @@ Public surface, argument order, output tuples and gradient contract follow the r
 :155-180), ``load_image_tiles_by_pos`` / ``merge_image_tiles_by_pos`` (:509-537) and the raw ``_C`` module.
 The two-stage split (per-Gaussian preprocess, then per-tile render, with the caller's all-to-all in between)
 is the reference's.  All compute runs in hand-written CUDA kernels behind the C ABI of
-``include/cgx_raster.h``; this file is autograd plumbing only.
+``include/cgx_raster.h``; the autograd nodes over it are C++ (``csrc/host.cpp``).  The Python nodes in this file do the
+same through the raw entry points of ``_C``; they serve per-stage profiling (``_C.PROFILE``), ``debug=True`` (which
+reads the device status after every operator) and empty inputs.
 """
 from typing import NamedTuple
 
@@ -15,6 +17,7 @@ import torch
 import torch.nn as nn
 
 from . import _C  # noqa: F401  (callers reach into diff_gaussian_rasterization._C directly)
+from . import _lib
 
 
 def cpu_deep_copy_tuple(input_tuple):
@@ -23,6 +26,8 @@ def cpu_deep_copy_tuple(input_tuple):
 
 # ----------------------------------------------------------------------------- preprocess
 def preprocess_gaussians(means3D, scales, rotations, sh, opacities, raster_settings, cuda_args):
+    if _C.PROFILE is None and not raster_settings.debug:
+        return tuple(_lib.host().preprocess(means3D, scales, rotations, sh, opacities, raster_settings))
     return _PreprocessGaussians.apply(means3D, scales, rotations, sh, opacities, raster_settings, cuda_args)
 
 
@@ -61,6 +66,10 @@ class _PreprocessGaussians(torch.autograd.Function):
 # ----------------------------------------------------------------------------- render
 def render_gaussians(means2D, means2D_abs, conic_opacity, rgb, all_map, depths, radii, compute_locally,
                      extended_compute_locally, raster_settings, cuda_args):
+    if _C.PROFILE is None and not raster_settings.debug and means2D.shape[0]:
+        local = extended_compute_locally if cuda_args["avoid_pixel_all2all"] else compute_locally
+        return tuple(_lib.host().render(means2D, means2D_abs, conic_opacity, rgb, all_map, depths, radii, local,
+                                        compute_locally, raster_settings, _C._stats(cuda_args)))
     return _RenderGaussians.apply(means2D, means2D_abs, conic_opacity, rgb, all_map, depths, radii, compute_locally,
                                   extended_compute_locally, raster_settings, cuda_args)
 

@@ -20,6 +20,9 @@ SOURCES = ["cabi.cu", "preprocess.cu", "binning.cu", "render.cu", "peer.cu", "lo
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-shared", "-Xcompiler", "-fPIC"]
 
+# C++ host path (csrc/host.cpp): autograd nodes over the same library
+HOST_SO = LIBDIR / "_cgx_host.so"
+
 CGX_OK, CGX_EINVAL, CGX_ENOMEM, CGX_ETIMEDOUT, CGX_ECUDA = 0, 22, 12, 110, 5
 
 
@@ -42,6 +45,31 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         print(" ".join(cmd), flush=True)
     subprocess.run(cmd, check=True)
     return SO
+
+
+def build_host(force: bool = False, verbose: bool = False) -> Path:
+    """Compile csrc/host.cpp against this interpreter's torch into lib/_cgx_host.so when out of date."""
+    import sysconfig
+
+    from torch.utils import cpp_extension as X
+    import torch
+
+    src = CSRC / "host.cpp"
+    newest = max(p.stat().st_mtime for p in (src, ROOT.parent / "include" / "cgx_raster.h"))
+    if not force and HOST_SO.exists() and HOST_SO.stat().st_mtime >= newest:
+        return HOST_SO
+    LIBDIR.mkdir(exist_ok=True)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    inc = list(X.include_paths()) + [sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    libs = X.library_paths() + [os.path.join(cuda, "lib64")]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_cgx_host",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd += [f"-isystem{i}" for i in inc] + [str(src)] + [f"-L{d}" for d in libs]
+    cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-lcudart", "-o", str(HOST_SO)]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    subprocess.run(cmd, check=True)
+    return HOST_SO
 
 
 _vp, _i, _f, _i64, _sz = C.c_void_p, C.c_int, C.c_float, C.c_int64, C.c_size_t
@@ -93,6 +121,7 @@ SIGNATURES = {
     "cgx_bin_workspace_bytes": (_sz, [_i]),
     "cgx_bin_count_scan": (_i, [_i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "cgx_bin_count_scan_depths": (_i, [_i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
+    "cgx_bin_count_scan_post": (_i, [_i, _i, _i] + [_vp] * 7 + [_sz, _vp, _vp]),
     "cgx_emit_keys": (_i, [_i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp]),
     "cgx_sort_workspace_bytes": (_sz, [_i64]),
     "cgx_sort_pairs": (_i, [_i64, _i, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
@@ -138,6 +167,28 @@ def lib():
             fn.argtypes = args
         _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The C++ host path, bound to the loaded library.  Raises if it has not been built: there is no fallback."""
+    global _host
+    if _host is None:
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries must be loaded first)
+
+        if not HOST_SO.exists():
+            raise ImportError(f"{HOST_SO} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`")
+        handle = lib()
+        spec = importlib.util.spec_from_file_location("_cgx_host", HOST_SO)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.bind({n: C.cast(getattr(handle, n), C.c_void_p).value for n in SIGNATURES}, CgxError)
+        _host = module
+    return _host
 
 
 class CgxError(RuntimeError):

@@ -62,7 +62,7 @@ int cgx_mark_visible(int P, const float* means3D, const float* viewmatrix, uint8
 int cgx_preprocess_fwd(int P, const float* means3D, const float* scales, float scale_modifier,
                        const float* rotations, const float* opacities, const float* viewmatrix,
                        const float* projmatrix, int W, int H, float tanfovx, float tanfovy,
-                       float* means2D, float* depths, int32_t* radii, float* cov3D, float* conic_opacity,
+                       float* means2D, float* depths, int32_t* radii, float* cov3D /* optional */, float* conic_opacity,
                        void* stream);
 
 /* RasterizeGaussiansfilterCUDA -> visible_filter -> filter_preprocessCUDA
@@ -384,6 +384,12 @@ int cgx_bin_count_scan(int P, int W, int H, const int32_t* radii, const float* m
 int cgx_bin_count_scan_depths(int P, int W, int H, const int32_t* radii, const float* means2D, const float* depths,
                               const uint8_t* compute_locally, uint32_t* tiles_touched, uint32_t* num_rendered3,
                               void* workspace, size_t workspace_bytes, void* stream);
+
+/* The same stage (P > 0, depths optional) for a host that waits for nothing but the count: the three words also go to
+ * page-locked host memory, behind them host_words4[3] = 1, which the caller clears before and watches after the call. */
+int cgx_bin_count_scan_post(int P, int W, int H, const int32_t* radii, const float* means2D, const float* depths,
+                            const uint8_t* compute_locally, uint32_t* tiles_touched, uint32_t* num_rendered3,
+                            void* workspace, size_t workspace_bytes, uint32_t* host_words4, void* stream);
 
 /* duplicateWithKeys (RAST/cuda_rasterizer/rasterizer_impl.cu:74-117): writes point_offsets u32 (P)
  * (inclusive sum, as the reference's GeometryState::point_offsets), keys u64 (R) =
