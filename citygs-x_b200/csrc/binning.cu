@@ -22,8 +22,7 @@ struct MaskBand {
     int valid, row0, row1, pad;
 };
 
-__global__ void __launch_bounds__(1024)
-analyse_mask_kernel(int gx, int gy, const uint8_t* __restrict__ local, MaskBand* __restrict__ band)
+__device__ __forceinline__ void analyse_mask(int gx, int gy, const uint8_t* __restrict__ local, MaskBand* __restrict__ band)
 {
     __shared__ int s_partial, s_first, s_last, s_full;
     if (threadIdx.x == 0) {
@@ -61,6 +60,12 @@ analyse_mask_kernel(int gx, int gy, const uint8_t* __restrict__ local, MaskBand*
         }
         *band = b;
     }
+}
+
+__global__ void __launch_bounds__(1024)
+analyse_mask_kernel(int gx, int gy, const uint8_t* __restrict__ local, MaskBand* __restrict__ band)
+{
+    analyse_mask(gx, gy, local, band);
 }
 
 __device__ __forceinline__ uint32_t count_local_tiles(const float2 xy, int radius, const uint8_t* __restrict__ local,
@@ -221,11 +226,10 @@ __device__ __forceinline__ uint32_t scan_row_inplace(uint32_t* __restrict__ row,
 // block_ranges (optional): per-CTA (min, max) depth bit patterns -> total_out[1], total_out[2].
 __global__ void __launch_bounds__(1024)
 scan_partials_kernel(int n, uint32_t* __restrict__ sums, uint32_t* __restrict__ total_out,
-                     const uint32_t* __restrict__ block_ranges, volatile uint32_t* host_words)
+                     const uint32_t* __restrict__ block_ranges)
 {
     const uint32_t total = scan_row_inplace(sums, n);
     if (threadIdx.x == 0) total_out[0] = total;
-    uint32_t all_min = 0xffffffffu, all_max = 0u;
     if (block_ranges) {
         __shared__ uint32_t s_min[32], s_max[32];
         uint32_t lo = 0xffffffffu, hi = 0u;
@@ -245,17 +249,9 @@ scan_partials_kernel(int n, uint32_t* __restrict__ sums, uint32_t* __restrict__ 
                 lo = min(lo, s_min[w]);
                 hi = max(hi, s_max[w]);
             }
-            total_out[1] = all_min = lo;
-            total_out[2] = all_max = hi;
+            total_out[1] = lo;
+            total_out[2] = hi;
         }
-    }
-    // the host watches the fourth word (see cgx_bin_count_scan_post)
-    if (host_words && threadIdx.x == 0) {
-        host_words[0] = total;
-        host_words[1] = all_min;
-        host_words[2] = all_max;
-        __threadfence_system();
-        host_words[3] = 1u;
     }
 }
 
@@ -762,6 +758,236 @@ tile_ranges_kernel(int64_t L, uint32_t T, const uint64_t* __restrict__ keys, uin
         }
     }
     if (idx == L - 1 && cur_ok) ranges[currtile].y = (uint32_t)L;
+}
+
+// ------------------------------------------------------------------------------------------------ lists per tile
+// The same lists without a global sort, for callers that need no sorted 64-bit keys: count the pairs of every tile,
+// scan the tiles, drop every pair (depth bits, Gaussian) into its tile's stretch in any order, and sort each stretch on
+// chip by (depth bits, Gaussian index), which is the order the stable sort of emitted keys leaves.  Four to six launches
+// instead of twenty, and 20 bytes per pair instead of 24 per pair and pass.
+
+constexpr int SMALL_TILE = 512, MID_TILE = 4096, LARGE_TILE = 16384;      // longest stretch of each kind of sorting CTA
+
+struct TileBins {
+    uint2* ranges;            // (T)
+    uint32_t* counts;         // (T) pairs of the tile, then its next free place
+    MaskBand* band;
+    uint32_t* tiles;          // (3, T) tiles of each kind
+    uint32_t* n_tiles;        // (3) how many
+};
+
+// One CTA: the mask as a band, and zeroed counts.
+__global__ void __launch_bounds__(1024)
+tile_bins_begin_kernel(int gx, int gy, const uint8_t* __restrict__ local, TileBins bins)
+{
+    for (int i = threadIdx.x; i < gx * gy; i += 1024) bins.counts[i] = 0;
+    if (threadIdx.x < 3) bins.n_tiles[threadIdx.x] = 0;
+    analyse_mask(gx, gy, local, bins.band);
+}
+
+// Calls f(tile) for every local tile of the splat.
+template <typename F>
+__device__ __forceinline__ void for_local_tiles(const float2 xy, int radius, const uint8_t* __restrict__ local, int gx,
+                                                int gy, const MaskBand band, F f)
+{
+    uint2 lo, hi;
+    get_rect(xy, radius, lo, hi, gx, gy);
+    const int y0 = band.valid ? max((int)lo.y, band.row0) : (int)lo.y;
+    const int y1 = band.valid ? min((int)hi.y, band.row1) : (int)hi.y;
+    for (int y = y0; y < y1; y++)
+        for (int x = lo.x; x < (int)hi.x; x++)
+            if (band.valid || local[y * gx + x]) f(y * gx + x);
+}
+
+__global__ void __launch_bounds__(CGX_BLOCK_SIZE)
+tile_bins_count_kernel(int P, int gx, int gy, const int* __restrict__ radii, const float2* __restrict__ means2D,
+                       const uint8_t* __restrict__ local, uint32_t* __restrict__ tiles_touched, const TileBins bins)
+{
+    const int i = blockIdx.x * CGX_BLOCK_SIZE + threadIdx.x;
+    if (i >= P) return;
+    const int r = radii[i];
+    uint32_t n = 0;
+    if (r > 0)
+        for_local_tiles(means2D[i], r, local, gx, gy, *bins.band, [&](int t) {
+            atomicAdd(&bins.counts[t], 1u);
+            n++;
+        });
+    tiles_touched[i] = n;
+}
+
+// One CTA: tile counts -> ranges and first free places, the lists of tiles by kind, and the words the host waits for:
+// pairs, longest stretch, tiles of each kind, flag.  A thread takes eight consecutive tiles, so a 3840x2160 grid is four
+// rounds.
+__global__ void __launch_bounds__(1024)
+tile_bins_scan_kernel(int T, TileBins bins, volatile uint32_t* host_words)
+{
+    __shared__ uint32_t s_warp[32], s_max[32], s_kind[3];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (t < 3) s_kind[t] = 0;
+    uint32_t carry = 0, longest = 0;
+    for (int start = 0; start < T; start += 8192) {
+        uint32_t v[8], sum = 0;
+        const int i0 = start + t * 8;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            v[k] = i0 + k < T ? bins.counts[i0 + k] : 0u;
+            sum += v[k];
+            longest = max(longest, v[k]);
+        }
+        const uint32_t incl = warp_incl_scan(sum);
+        __syncthreads();                       // the previous round has read s_warp
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        uint32_t before = 0, total = 0;
+#pragma unroll
+        for (int w = 0; w < 32; w++) {
+            if (w < warp) before += s_warp[w];
+            total += s_warp[w];
+        }
+        uint32_t at = carry + before + incl - sum;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            if (i0 + k >= T) break;
+            bins.ranges[i0 + k] = make_uint2(at, at + v[k]);
+            bins.counts[i0 + k] = at;
+            at += v[k];
+            if (v[k]) {
+                const int kind = v[k] <= SMALL_TILE ? 0 : v[k] <= MID_TILE ? 1 : 2;
+                bins.tiles[(size_t)kind * T + atomicAdd(&s_kind[kind], 1u)] = i0 + k;
+            }
+        }
+        carry += total;
+    }
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if (lane == 0) s_max[warp] = longest;
+    __syncthreads();
+    if (t == 0) {
+        for (int w = 1; w < 32; w++) longest = max(longest, s_max[w]);
+        for (int k = 0; k < 3; k++) bins.n_tiles[k] = s_kind[k];
+        if (host_words) {
+            host_words[0] = carry;
+            host_words[1] = longest;
+            for (int k = 0; k < 3; k++) host_words[2 + k] = s_kind[k];
+            __threadfence_system();
+            host_words[5] = 1u;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(CGX_BLOCK_SIZE)
+tile_bins_fill_kernel(int P, int gx, int gy, const int* __restrict__ radii, const float2* __restrict__ means2D,
+                      const float* __restrict__ depths, const uint8_t* __restrict__ local, const TileBins bins,
+                      uint64_t* __restrict__ pairs, uint32_t capacity)
+{
+    const int i = blockIdx.x * CGX_BLOCK_SIZE + threadIdx.x;
+    if (i >= P) return;
+    const int r = radii[i];
+    if (r <= 0) return;
+    const uint64_t pair = ((uint64_t)__float_as_uint(depths[i]) << 32) | (uint32_t)i;
+    for_local_tiles(means2D[i], r, local, gx, gy, *bins.band, [&](int t) {
+        const uint32_t at = atomicAdd(&bins.counts[t], 1u);
+        if (at < capacity) pairs[at] = pair;
+    });
+}
+
+// Sorts one tile's stretch per CTA: bucket sort by depth (as many buckets as there is room for pairs, spread over the
+// stretch's depth range), then every pair finds its place among the few of its bucket.  Where depths crowd into few
+// buckets that search would be quadratic: such a stretch is sorted by a bitonic network instead.
+constexpr uint32_t CROWDED = 96;      // pairs of one bucket from which the network is the cheaper way
+template <int THREADS, int MOST>
+__global__ void __launch_bounds__(THREADS)
+tile_sort_kernel(const uint32_t* __restrict__ tiles, const uint2* __restrict__ ranges, const uint64_t* __restrict__ pairs,
+                 uint32_t* __restrict__ list)
+{
+    constexpr int ITEMS = MOST / THREADS, WARPS = THREADS / 32, PER = MOST / 2 / THREADS;   // MOST / 2 buckets
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint64_t* s_pair = reinterpret_cast<uint64_t*>(smem_raw);
+    uint32_t* s_start = reinterpret_cast<uint32_t*>(s_pair + MOST);      // counts, then first places
+    __shared__ uint32_t s_red[2][WARPS];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint2 range = ranges[tiles[blockIdx.x]];
+    const int n = range.y - range.x;
+    uint64_t item[ITEMS];
+    uint32_t lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) {
+        const int i = k * THREADS + t;
+        if (i < n) {
+            item[k] = pairs[range.x + i];
+            const uint32_t d = (uint32_t)(item[k] >> 32);
+            lo = min(lo, d);
+            hi = max(hi, d);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < PER; k++) s_start[k * THREADS + t] = 0;
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) s_red[0][warp] = lo, s_red[1][warp] = hi;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < WARPS; w++) lo = min(lo, s_red[0][w]), hi = max(hi, s_red[1][w]);
+    // bucket of a depth: rounding is monotone, so a smaller depth never falls into a later bucket
+    const float scale = (float)(MOST / 2) / ((float)(hi - lo) + 1.f);
+    auto bucket_of = [&](uint64_t p) { return min((int)((float)((uint32_t)(p >> 32) - lo) * scale), MOST / 2 - 1); };
+    uint16_t rank[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++)
+        if (k * THREADS + t < n) rank[k] = (uint16_t)atomicAdd(&s_start[bucket_of(item[k])], 1u);
+    __syncthreads();
+    uint32_t c[PER], sum = 0, most = 0;
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        c[k] = s_start[t * PER + k];
+        sum += c[k];
+        most = max(most, c[k]);
+    }
+    const uint32_t incl = warp_incl_scan(sum);
+    if (lane == 31) s_red[0][warp] = incl;
+    const bool crowded = __syncthreads_or(most > CROWDED);
+    uint32_t at = incl - sum;
+#pragma unroll
+    for (int w = 0; w < WARPS; w++)
+        if (w < warp) at += s_red[0][w];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        s_start[t * PER + k] = at;
+        at += c[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++)
+        if (k * THREADS + t < n) s_pair[s_start[bucket_of(item[k])] + rank[k]] = item[k];
+    if (!crowded) {
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            if (k * THREADS + t >= n) continue;
+            const int b = bucket_of(item[k]);
+            const uint32_t first = s_start[b], last = b + 1 < MOST / 2 ? s_start[b + 1] : (uint32_t)n;
+            uint32_t place = first;
+            for (uint32_t j = first; j < last; j++) place += s_pair[j] < item[k];
+            list[range.x + place] = (uint32_t)item[k];
+        }
+        return;
+    }
+    int size = 2;
+    while (size < n) size <<= 1;
+    for (int i = n + t; i < size; i += THREADS) s_pair[i] = ~0ull;
+    for (int k = 2; k <= size; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            __syncthreads();
+            for (int i = t; i < size / 2; i += THREADS) {
+                const int a = 2 * i - (i & (j - 1)), b = a + j;
+                const uint64_t x = s_pair[a], y = s_pair[b];
+                if ((x > y) == ((a & k) == 0)) {
+                    s_pair[a] = y;
+                    s_pair[b] = x;
+                }
+            }
+        }
+    __syncthreads();
+    for (int i = t; i < n; i += THREADS) list[range.x + i] = (uint32_t)s_pair[i];
 }
 
 // ------------------------------------------------------------------------------------------------ distribution
@@ -1308,15 +1534,10 @@ extern "C" size_t cgx_bin_workspace_bytes(int P)
 
 static int bin_count_scan(int P, int W, int H, const int32_t* radii, const float* means2D, const float* depths,
                           const uint8_t* compute_locally, uint32_t* tiles_touched, uint32_t* num_rendered,
-                          void* workspace, size_t workspace_bytes, void* stream, uint32_t* host_words = nullptr)
+                          void* workspace, size_t workspace_bytes, void* stream)
 {
     if (P < 0 || W <= 0 || H <= 0 || !num_rendered) return CGX_EINVAL;
     cudaStream_t st = (cudaStream_t)stream;
-    void* mapped = nullptr;
-    if (host_words) {       // fails for pageable memory: the caller must pass page-locked memory
-        cudaError_t e = cudaHostGetDevicePointer(&mapped, host_words, 0);
-        if (e != cudaSuccess || !mapped) { (void)cudaGetLastError(); return CGX_EINVAL; }
-    }
     if (P == 0) {
         cudaError_t e = cudaMemsetAsync(num_rendered, 0, (depths ? 3 : 1) * sizeof(uint32_t), st);
         if (e != cudaSuccess) { set_cuda_error(e); return CGX_ECUDA; }
@@ -1334,7 +1555,7 @@ static int bin_count_scan(int P, int W, int H, const int32_t* radii, const float
     const int vec_ok = aligned16(radii) && aligned16(means2D) && aligned16(tiles_touched) && (!depths || aligned16(depths));
     tile_count_kernel<<<nblocks, CGX_BLOCK_SIZE, 0, st>>>(P, gx, gy, radii, (const float2*)means2D, compute_locally,
                                                           tiles_touched, sums, band, depths, block_ranges, vec_ok);
-    scan_partials_kernel<<<1, 1024, 0, st>>>(nblocks, sums, num_rendered, block_ranges, (volatile uint32_t*)mapped);
+    scan_partials_kernel<<<1, 1024, 0, st>>>(nblocks, sums, num_rendered, block_ranges);
     return check_launch(3);
 }
 
@@ -1353,16 +1574,6 @@ extern "C" int cgx_bin_count_scan_depths(int P, int W, int H, const int32_t* rad
     if (P > 0 && !depths) return CGX_EINVAL;
     return bin_count_scan(P, W, H, radii, means2D, depths, compute_locally, tiles_touched, num_rendered3, workspace,
                           workspace_bytes, stream);
-}
-
-extern "C" int cgx_bin_count_scan_post(int P, int W, int H, const int32_t* radii, const float* means2D,
-                                       const float* depths, const uint8_t* compute_locally, uint32_t* tiles_touched,
-                                       uint32_t* num_rendered3, void* workspace, size_t workspace_bytes,
-                                       uint32_t* host_words4, void* stream)
-{
-    if (P <= 0 || !host_words4) return CGX_EINVAL;
-    return bin_count_scan(P, W, H, radii, means2D, depths, compute_locally, tiles_touched, num_rendered3, workspace,
-                          workspace_bytes, stream, host_words4);
 }
 
 extern "C" int cgx_emit_keys(int P, int W, int H, const int32_t* radii, const float* means2D, const float* depths,
@@ -1545,6 +1756,96 @@ extern "C" int cgx_sort_pairs_pingpong(int64_t n, int end_bit, int low_bits, uin
         return CGX_ENOMEM;
     return sort_passes_run(g_sort_variant, n, end_bit, low_bits, keys_a, values_a, keys_b, values_b, workspace,
                            workspace_bytes, wait_limit_cycles, (cudaStream_t)stream);
+}
+
+static size_t tile_bins_carve(int W, int H, void* workspace, TileBins* b)
+{
+    const size_t T = (size_t)((W + CGX_BLOCK_X - 1) / CGX_BLOCK_X) * ((H + CGX_BLOCK_Y - 1) / CGX_BLOCK_Y);
+    char* p = (char*)workspace;
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        char* r = p ? p + at : nullptr;
+        at += align_up(bytes, 256);
+        return r;
+    };
+    TileBins t;
+    t.ranges = (uint2*)take(T * sizeof(uint2));
+    t.counts = (uint32_t*)take(T * sizeof(uint32_t));
+    t.band = (MaskBand*)take(sizeof(MaskBand));
+    t.n_tiles = (uint32_t*)take(3 * sizeof(uint32_t));
+    t.tiles = (uint32_t*)take(3 * T * sizeof(uint32_t));
+    if (b) *b = t;
+    return at;
+}
+
+extern "C" size_t cgx_tile_bins_workspace_bytes(int W, int H)
+{
+    return W > 0 && H > 0 ? tile_bins_carve(W, H, nullptr, nullptr) : 0;
+}
+extern "C" int cgx_tile_bins_longest(void) { return LARGE_TILE; }
+
+extern "C" int cgx_tile_bins_count(int P, int W, int H, const int32_t* radii, const float* means2D,
+                                   const uint8_t* compute_locally, uint32_t* tiles_touched, void* workspace,
+                                   size_t workspace_bytes, uint32_t* host_words6, void* stream)
+{
+    if (P <= 0 || W <= 0 || H <= 0 || !radii || !means2D || ((uintptr_t)means2D & 7) || !compute_locally ||
+        !tiles_touched || !workspace || ((uintptr_t)workspace & 7))
+        return CGX_EINVAL;
+    if (workspace_bytes < cgx_tile_bins_workspace_bytes(W, H)) return CGX_ENOMEM;
+    void* mapped = nullptr;
+    if (host_words6) {       // fails for pageable memory: the caller must pass page-locked memory
+        cudaError_t e = cudaHostGetDevicePointer(&mapped, host_words6, 0);
+        if (e != cudaSuccess || !mapped) { (void)cudaGetLastError(); return CGX_EINVAL; }
+    }
+    const int gx = (W + CGX_BLOCK_X - 1) / CGX_BLOCK_X, gy = (H + CGX_BLOCK_Y - 1) / CGX_BLOCK_Y;
+    cudaStream_t st = (cudaStream_t)stream;
+    TileBins b;
+    tile_bins_carve(W, H, workspace, &b);
+    tile_bins_begin_kernel<<<1, 1024, 0, st>>>(gx, gy, compute_locally, b);
+    tile_bins_count_kernel<<<(P + CGX_BLOCK_SIZE - 1) / CGX_BLOCK_SIZE, CGX_BLOCK_SIZE, 0, st>>>(
+        P, gx, gy, radii, (const float2*)means2D, compute_locally, tiles_touched, b);
+    tile_bins_scan_kernel<<<1, 1024, 0, st>>>(gx * gy, b, (volatile uint32_t*)mapped);
+    return check_launch(3);
+}
+
+template <int THREADS, int MOST>
+static int launch_tile_sort(int n_tiles, const uint32_t* tiles, const uint2* ranges, const uint64_t* pairs,
+                            uint32_t* list, cudaStream_t st)
+{
+    constexpr int smem = MOST * sizeof(uint64_t) + MOST / 2 * sizeof(uint32_t);
+    cudaError_t e = cudaFuncSetAttribute(tile_sort_kernel<THREADS, MOST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) { set_cuda_error(e); return CGX_ECUDA; }
+    tile_sort_kernel<THREADS, MOST><<<n_tiles, THREADS, smem, st>>>(tiles, ranges, pairs, list);
+    return check_launch();
+}
+
+extern "C" int cgx_tile_bins_sort(int P, int W, int H, const int32_t* radii, const float* means2D, const float* depths,
+                                  const uint8_t* compute_locally, const uint32_t* host_words6, void* workspace,
+                                  size_t workspace_bytes, uint64_t* pairs, uint32_t* point_list, void* stream)
+{
+    if (P <= 0 || W <= 0 || H <= 0 || !radii || !means2D || ((uintptr_t)means2D & 7) || !depths || !compute_locally ||
+        !host_words6 || !workspace || ((uintptr_t)workspace & 7))
+        return CGX_EINVAL;
+    if (workspace_bytes < cgx_tile_bins_workspace_bytes(W, H)) return CGX_ENOMEM;
+    const uint32_t R = host_words6[0];
+    if (R == 0) return CGX_OK;
+    if (!pairs || !point_list) return CGX_EINVAL;
+    if (host_words6[1] > (uint32_t)LARGE_TILE) return CGX_ENOMEM;
+    const int gx = (W + CGX_BLOCK_X - 1) / CGX_BLOCK_X, gy = (H + CGX_BLOCK_Y - 1) / CGX_BLOCK_Y, T = gx * gy;
+    cudaStream_t st = (cudaStream_t)stream;
+    TileBins b;
+    tile_bins_carve(W, H, workspace, &b);
+    tile_bins_fill_kernel<<<(P + CGX_BLOCK_SIZE - 1) / CGX_BLOCK_SIZE, CGX_BLOCK_SIZE, 0, st>>>(
+        P, gx, gy, radii, (const float2*)means2D, depths, compute_locally, b, pairs, R);
+    int s = check_launch();
+    // long stretches first: their CTAs take longest
+    if (s == CGX_OK && host_words6[4])
+        s = launch_tile_sort<1024, LARGE_TILE>(host_words6[4], b.tiles + 2 * (size_t)T, b.ranges, pairs, point_list, st);
+    if (s == CGX_OK && host_words6[3])
+        s = launch_tile_sort<256, MID_TILE>(host_words6[3], b.tiles + T, b.ranges, pairs, point_list, st);
+    if (s == CGX_OK && host_words6[2])
+        s = launch_tile_sort<64, SMALL_TILE>(host_words6[2], b.tiles, b.ranges, pairs, point_list, st);
+    return s;
 }
 
 extern "C" int cgx_tile_ranges(int64_t n, int T, const uint64_t* keys_sorted, uint32_t* ranges, void* stream)

@@ -26,7 +26,8 @@ namespace {
 #define CGX_FUNCTIONS(X)                                                                                             \
     X(cgx_preprocess_fwd) X(cgx_preprocess_bwd) X(cgx_preprocess_fwd_batched_planes) X(cgx_preprocess_bwd_batched_planes) \
     X(cgx_all_map_fwd) X(cgx_all_map_bwd) X(cgx_strip_loss_fwd) X(cgx_strip_loss_bwd) X(cgx_depth_normal_fwd)        \
-    X(cgx_depth_normal_bwd) X(cgx_bin_workspace_bytes) X(cgx_bin_count_scan_post) X(cgx_emit_keys)                   \
+    X(cgx_depth_normal_bwd) X(cgx_bin_workspace_bytes) X(cgx_bin_count_scan) X(cgx_emit_keys)                        \
+    X(cgx_tile_bins_workspace_bytes) X(cgx_tile_bins_longest) X(cgx_tile_bins_count) X(cgx_tile_bins_sort)          \
     X(cgx_sort_workspace_bytes) X(cgx_sort_passes) X(cgx_sort_pairs_pingpong) X(cgx_tile_ranges) X(cgx_higher_msb)   \
     X(cgx_render_records_bytes) X(cgx_render_fwd) X(cgx_render_bwd_workspace_bytes) X(cgx_render_bwd_table)
 struct Library {
@@ -128,42 +129,25 @@ struct Carver {
     }
 };
 struct GeometryLayout {
-    size_t tiles_touched, scan, scan_bytes, offsets, num_rendered, records, total;
-    explicit GeometryLayout(int64_t P)
+    size_t tiles_touched, bins, bins_bytes, records, total;
+    GeometryLayout(int64_t P, int W, int H)
     {
         Carver c;
         tiles_touched = c.add(4 * P);
-        scan_bytes = L.cgx_bin_workspace_bytes((int)P);
-        scan = c.add(scan_bytes);
-        offsets = c.add(4 * P);
-        num_rendered = c.add(4 * 32);
+        bins_bytes = L.cgx_tile_bins_workspace_bytes(W, H);      // its first words are the tile ranges
+        bins = c.add(bins_bytes);
         records = c.add(L.cgx_render_records_bytes((int)P));
         total = c.size + 128;
     }
 };
-struct BinningLayout {
-    size_t list, list_unsorted, keys, keys_unsorted, sort, sort_bytes, total;
-    explicit BinningLayout(int64_t R)
-    {
-        Carver c;
-        list = c.add(4 * R);
-        list_unsorted = c.add(4 * R);
-        keys = c.add(8 * R);
-        keys_unsorted = c.add(8 * R);
-        sort_bytes = L.cgx_sort_workspace_bytes(R);
-        sort = c.add(sort_bytes);
-        total = c.size + 128;
-    }
-};
 struct ImageLayout {
-    size_t accum_alpha, n_contrib, n_contrib2loss, ranges, total;
-    ImageLayout(int64_t N, int64_t T)
+    size_t accum_alpha, n_contrib, n_contrib2loss, total;
+    explicit ImageLayout(int64_t N)
     {
         Carver c;
         accum_alpha = c.add(4 * N);
         n_contrib = c.add(4 * N);
         n_contrib2loss = c.add(4 * N);
-        ranges = c.add(8 * T);
         total = c.size + 128;
     }
 };
@@ -223,11 +207,13 @@ void report(const Stats& stats, const char* key, std::shared_ptr<EventMs> ms)
 }
 
 // ---------------------------------------------------------------------------------------------- pair counts
-// The counting stage leaves (pairs, smallest and largest depth word) in page-locked memory, with a flag behind them that
-// the host watches: neither a copy nor an event stands between the kernel and the launches that need the count.
+// The counting stage leaves the number of pairs and what the tiles' lists look like in page-locked memory, with a flag
+// behind them that the host watches: neither a copy nor an event stands between the kernel and the launches that need them.
 constexpr int SLOTS = 256;
 struct Slot {
-    volatile uint32_t pairs, dmin, dmax, flag;
+    uint32_t word[5];          // see cgx_tile_bins_count
+    volatile uint32_t flag;
+    uint32_t pad[2];
 };
 Slot* slots()
 {
@@ -243,7 +229,7 @@ struct Count {
     Tensor geom;
     int slot = -1;
     cudaStream_t stream = nullptr;
-    bool ranged = false;
+    uint32_t word[6];
     Tensor keep[3];            // a prefetched count's inputs: their addresses stay taken
 };
 std::mutex slot_lock;
@@ -266,26 +252,22 @@ void give_slot(int s)
     free_slots.push_back(s);
 }
 
-Count start_count(int64_t P, int W, int H, const Tensor& means2D, const Tensor& radii, const Tensor& depths,
-                  const Tensor& local)
+Count start_count(int64_t P, int W, int H, const Tensor& means2D, const Tensor& radii, const Tensor& local)
 {
-    const GeometryLayout gl(P);
+    const GeometryLayout gl(P, W, H);
     Count c;
     c.geom = bytes_like(gl.total, means2D);
     c.slot = take_slot();
     c.stream = at::cuda::getCurrentCUDAStream().stream();
-    c.ranged = depths.defined();
     Slot& s = slots()[c.slot];
     s.flag = 0;
-    check(L.cgx_bin_count_scan_post((int)P, W, H, i32(radii), f32(means2D), f32(depths),
-                                    static_cast<uint8_t*>(local.data_ptr()), at_offset<uint32_t>(c.geom, gl.tiles_touched),
-                                    at_offset<uint32_t>(c.geom, gl.num_rendered), at_offset<void>(c.geom, gl.scan),
-                                    gl.scan_bytes, const_cast<uint32_t*>(&s.pairs), c.stream),
-          "cgx_bin_count_scan");
+    check(L.cgx_tile_bins_count((int)P, W, H, i32(radii), f32(means2D), static_cast<uint8_t*>(local.data_ptr()),
+                                at_offset<uint32_t>(c.geom, gl.tiles_touched), at_offset<void>(c.geom, gl.bins),
+                                gl.bins_bytes, s.word, c.stream), "cgx_tile_bins_count");
     return c;
 }
 // Waits for the count; gives the slot back.
-void finish_count(Count& c, int64_t& R, int& low_bits)
+void finish_count(Count& c)
 {
     Slot& s = slots()[c.slot];
     const auto t0 = std::chrono::steady_clock::now();
@@ -294,15 +276,12 @@ void finish_count(Count& c, int64_t& R, int& low_bits)
         if (++spins % 1024 == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(2)) {
             // a long queue in front of it, or an error: let the driver wait, and say so if there was one
             const cudaError_t e = cudaStreamSynchronize(c.stream);
-            if (e != cudaSuccess) throw std::runtime_error(std::string("cgx_bin_count_scan: ") + cudaGetErrorString(e));
-            if (!s.flag) throw std::runtime_error("cgx_bin_count_scan: the pair count did not arrive");
+            if (e != cudaSuccess) throw std::runtime_error(std::string("cgx_tile_bins_count: ") + cudaGetErrorString(e));
+            if (!s.flag) throw std::runtime_error("cgx_tile_bins_count: the pair count did not arrive");
         }
     }
     std::atomic_thread_fence(std::memory_order_acquire);
-    R = s.pairs;
-    const uint32_t lo = s.dmin, hi = s.dmax;
-    low_bits = 32;
-    if (c.ranged && lo <= hi) low_bits = lo == hi ? 1 : 32 - __builtin_clz(lo ^ hi);
+    for (int k = 0; k < 5; k++) c.word[k] = s.word[k];
     give_slot(c.slot);
     c.slot = -1;
 }
@@ -329,8 +308,7 @@ bool find_prefetched(Count& c, const Tensor& means2D, const Tensor& radii, const
     return true;
 }
 
-void prefetch(int H, int W, const Tensor& means2D_, const Tensor& radii_, const Tensor& local_,
-              const c10::optional<Tensor>& depths_)
+void prefetch(int H, int W, const Tensor& means2D_, const Tensor& radii_, const Tensor& local_)
 {
     const Tensor means2D = cuda_f32(means2D_, "means2D"), radii = cuda_any(radii_, "radii"),
                  local = cuda_any(local_, "compute_locally");
@@ -339,41 +317,32 @@ void prefetch(int H, int W, const Tensor& means2D_, const Tensor& radii_, const 
     const c10::cuda::CUDAGuard guard(means2D.device());
     std::lock_guard<std::mutex> g(prefetch_lock);
     if (prefetched.size() >= PREFETCH_MOST) {              // counts nobody picked up
-        for (auto& e : prefetched) {
-            int64_t R;
-            int bits;
-            finish_count(e.second, R, bits);
-        }
+        for (auto& e : prefetched) finish_count(e.second);
         prefetched.clear();
     }
     const PrefetchKey key = prefetch_key(means2D, radii, local, H, W);
     const auto old = prefetched.find(key);
     if (old != prefetched.end()) {
-        int64_t R;
-        int bits;
-        finish_count(old->second, R, bits);
+        finish_count(old->second);
         prefetched.erase(old);
     }
-    Count c = start_count(P, W, H, means2D, radii, depths_ ? cuda_f32(*depths_, "depths") : Tensor(), local);
+    Count c = start_count(P, W, H, means2D, radii, local);
     c.keep[0] = means2D;
     c.keep[1] = radii;
     c.keep[2] = local;
     prefetched.emplace(key, std::move(c));
 }
 
-// (geometry buffer, pairs, varying depth bits) of a count started ahead, or None.
+// The pairs of a count started ahead, or None.
 py::object take_prefetched(int H, int W, const Tensor& means2D, const Tensor& radii, const Tensor& local)
 {
     Count c;
-    int64_t R = 0;
-    int bits = 32;
     {
         py::gil_scoped_release nogil;
-        if (!find_prefetched(c, means2D, radii, local, H, W)) c.slot = -1;
-        else finish_count(c, R, bits);
+        if (find_prefetched(c, means2D, radii, local, H, W)) finish_count(c);
     }
     if (!c.geom.defined()) return py::none();
-    return py::make_tuple(c.geom, R, bits);
+    return py::int_(c.word[0]);
 }
 size_t prefetched_counts()
 {
@@ -383,12 +352,37 @@ size_t prefetched_counts()
 
 // ---------------------------------------------------------------------------------------------- render
 struct RenderState {
-    int64_t P, R;
+    int64_t P;
     int H, W;
     float tanfovx, tanfovy;
     bool geo;
     Stats stats;
 };
+
+// Lists with a tile longer than the per-tile sort takes: emission, global sort, ranges.
+void sort_globally(int64_t P, int64_t R, int W, int H, int64_t T, const Tensor& radii, const Tensor& means2D,
+                   const Tensor& depths, uint8_t* local, uint32_t* tiles, uint32_t* list, uint32_t* ranges, cudaStream_t st)
+{
+    Carver c;
+    const size_t scan_bytes = L.cgx_bin_workspace_bytes((int)P), sort_bytes = L.cgx_sort_workspace_bytes(R);
+    const size_t scan = c.add(scan_bytes), words = c.add(128), offsets = c.add(4 * P), list_b = c.add(4 * R),
+                 keys_a = c.add(8 * R), keys_b = c.add(8 * R), sort = c.add(sort_bytes);
+    const Tensor buf = bytes_like(c.size + 128, means2D);
+    const int bit = (int)L.cgx_higher_msb((uint32_t)T);
+    // the sort ping-pongs: the pairs are emitted where the last pass lands in `list`
+    const bool even = L.cgx_sort_passes(32 + bit) % 2 == 0;
+    uint32_t* v[2] = {list, at_offset<uint32_t>(buf, list_b)};
+    uint64_t* k[2] = {at_offset<uint64_t>(buf, keys_a), at_offset<uint64_t>(buf, keys_b)};
+    const int first = even ? 0 : 1;
+    check(L.cgx_bin_count_scan((int)P, W, H, i32(radii), f32(means2D), local, tiles, at_offset<uint32_t>(buf, words),
+                               at_offset<void>(buf, scan), scan_bytes, st), "cgx_bin_count_scan");
+    check(L.cgx_emit_keys((int)P, W, H, i32(radii), f32(means2D), f32(depths), tiles, local,
+                          at_offset<uint32_t>(buf, offsets), k[first], v[first], R, at_offset<void>(buf, scan), st),
+          "cgx_emit_keys");
+    check(L.cgx_sort_pairs_pingpong(R, 32 + bit, 32, k[first], v[first], k[1 - first], v[1 - first],
+                                    at_offset<void>(buf, sort), sort_bytes, 0, st), "cgx_sort_pairs");
+    check(L.cgx_tile_ranges(R, (int)T, k[0], ranges, st), "cgx_tile_ranges");
+}
 
 struct Render : torch::autograd::Function<Render> {
     static variable_list forward(AutogradContext* ctx, const Tensor& means2D_, const c10::optional<Tensor>& means2D_abs,
@@ -414,39 +408,33 @@ struct Render : torch::autograd::Function<Render> {
 
         Count count;
         if (!find_prefetched(count, means2D, radii, local, H, W))
-            count = start_count(P, W, H, means2D, radii, depths, local);
+            count = start_count(P, W, H, means2D, radii, local);
         // allocated while the count is on its way
-        const GeometryLayout gl(P);
-        const ImageLayout il(HW, T);
+        const GeometryLayout gl(P, W, H);
+        const ImageLayout il(HW);
         const Tensor n_render = empty_i32({T}, means2D), n_consider = empty_i32({T}, means2D),
                      n_contrib = empty_i32({T}, means2D), observe = empty_i32({P}, means2D),
                      color = empty_f32({3, H, W}, means2D), out_map = empty_f32({5, H, W}, means2D),
                      depth = empty_f32({1, H, W}, means2D), img = bytes_like(il.total, means2D);
         std::shared_ptr<EventMs> ms = stats ? std::make_shared<EventMs>() : nullptr;
-        const int bit = (int)L.cgx_higher_msb((uint32_t)T);
-        int64_t R;
-        int low_bits;
-        finish_count(count, R, low_bits);
+        finish_count(count);
 
-        const BinningLayout bl(R);
-        const Tensor bin = bytes_like(bl.total, means2D);
-        if (ms) cudaEventRecord(ms->a, st);
-        // the sort ping-pongs between the two key/value arrays: the pairs are emitted into whichever array makes the last
-        // pass land in keys / list
-        const bool even = L.cgx_sort_passes(low_bits + bit) % 2 == 0;
-        uint64_t* keys[2] = {at_offset<uint64_t>(bin, bl.keys), at_offset<uint64_t>(bin, bl.keys_unsorted)};
-        uint32_t* list[2] = {at_offset<uint32_t>(bin, bl.list), at_offset<uint32_t>(bin, bl.list_unsorted)};
-        const int first = even ? 0 : 1;
+        const int64_t R = count.word[0];
+        const Tensor list = at::empty({R}, means2D.options().dtype(at::kInt).requires_grad(false));
         uint32_t* tiles = at_offset<uint32_t>(count.geom, gl.tiles_touched);
+        uint32_t* ranges = at_offset<uint32_t>(count.geom, gl.bins);
         uint8_t* loc = static_cast<uint8_t*>(local.data_ptr());
-        uint32_t* ranges = at_offset<uint32_t>(img, il.ranges);
-        check(L.cgx_emit_keys((int)P, W, H, i32(radii), f32(means2D), f32(depths), tiles, loc,
-                              at_offset<uint32_t>(count.geom, gl.offsets), keys[first], list[first], R,
-                              at_offset<void>(count.geom, gl.scan), st), "cgx_emit_keys");
-        check(L.cgx_sort_pairs_pingpong(R, 32 + bit, low_bits, keys[first], list[first], keys[1 - first], list[1 - first],
-                                        at_offset<void>(bin, bl.sort), bl.sort_bytes, 0, st), "cgx_sort_pairs");
-        check(L.cgx_tile_ranges(R, (int)T, keys[0], ranges, st), "cgx_tile_ranges");
-        check(L.cgx_render_fwd((int)P, W, H, s.tanfovx, s.tanfovy, ranges, list[0], i32(radii), f32(means2D), f32(rgb),
+        uint32_t* ids = static_cast<uint32_t*>(list.data_ptr());
+        if (ms) cudaEventRecord(ms->a, st);
+        if (count.word[1] <= (uint32_t)L.cgx_tile_bins_longest()) {
+            const Tensor pairs = bytes_like(8 * R, means2D);
+            check(L.cgx_tile_bins_sort((int)P, W, H, i32(radii), f32(means2D), f32(depths), loc, count.word,
+                                       at_offset<void>(count.geom, gl.bins), gl.bins_bytes,
+                                       static_cast<uint64_t*>(pairs.data_ptr()), ids, st), "cgx_tile_bins_sort");
+        } else {
+            sort_globally(P, R, W, H, T, radii, means2D, depths, loc, tiles, ids, ranges, st);
+        }
+        check(L.cgx_render_fwd((int)P, W, H, s.tanfovx, s.tanfovy, ranges, ids, i32(radii), f32(means2D), f32(rgb),
                                f32(all_map), f32(conic), loc, f32(bg), s.geo, at_offset<void>(count.geom, gl.records),
                                at_offset<float>(img, il.accum_alpha), at_offset<uint32_t>(img, il.n_contrib),
                                at_offset<uint32_t>(img, il.n_contrib2loss), f32(color), i32(observe), f32(out_map),
@@ -457,8 +445,8 @@ struct Render : torch::autograd::Function<Render> {
         }
         ctx->set_materialize_grads(false);
         ctx->mark_non_differentiable({n_render, n_consider, n_contrib, observe});
-        ctx->save_for_backward({out_map, count.geom, bin, img, cuda_any(local_bwd, "compute_locally"), bg});
-        keep(ctx, RenderState{P, R, H, W, s.tanfovx, s.tanfovy, s.geo, stats});
+        ctx->save_for_backward({out_map, count.geom, list, img, cuda_any(local_bwd, "compute_locally"), bg});
+        keep(ctx, RenderState{P, H, W, s.tanfovx, s.tanfovy, s.geo, stats});
         return {color, n_render, n_consider, n_contrib, observe, out_map, depth};
     }
 
@@ -466,7 +454,7 @@ struct Render : torch::autograd::Function<Render> {
     {
         const RenderState& s = kept<RenderState>(ctx);
         const variable_list saved = ctx->get_saved_variables();
-        const Tensor &out_map = saved[0], &geom = saved[1], &bin = saved[2], &img = saved[3], &local = saved[4], &bg = saved[5];
+        const Tensor &out_map = saved[0], &geom = saved[1], &list = saved[2], &img = saved[3], &local = saved[4], &bg = saved[5];
         const c10::cuda::CUDAGuard guard(out_map.device());
         const cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
         auto cotangent = [&](const Tensor& t, int n, const char* name, bool needed) {
@@ -475,18 +463,17 @@ struct Render : torch::autograd::Function<Render> {
         };
         const Tensor d_color = cotangent(g[0], 3, "dL_dout_color", true), d_map = cotangent(g[5], 5, "dL_dout_all_map", s.geo),
                      d_depth = cotangent(g[6], 1, "dL_dout_plane_depth", s.geo);
-        const int64_t P = s.P, HW = (int64_t)s.H * s.W, T = (int64_t)((s.W + 15) / 16) * ((s.H + 15) / 16);
-        const GeometryLayout gl(P);
-        const BinningLayout bl(s.R);
-        const ImageLayout il(HW, T);
+        const int64_t P = s.P, HW = (int64_t)s.H * s.W;
+        const GeometryLayout gl(P, s.W, s.H);
+        const ImageLayout il(HW);
         const Tensor m2 = empty_f32({P, 2}, out_map), abs2 = empty_f32({P, 3}, out_map), co = empty_f32({P, 4}, out_map),
                      rgb = empty_f32({P, 3}, out_map), am = empty_f32({P, 5}, out_map);
         const size_t ws_bytes = L.cgx_render_bwd_workspace_bytes((int)P);
         const Tensor ws = bytes_like(ws_bytes, out_map);
         std::shared_ptr<EventMs> ms = s.stats ? std::make_shared<EventMs>() : nullptr;
         if (ms) cudaEventRecord(ms->a, st);
-        check(L.cgx_render_bwd_table((int)P, s.W, s.H, s.tanfovx, s.tanfovy, at_offset<uint32_t>(img, il.ranges),
-                                     at_offset<uint32_t>(bin, bl.list), f32(bg), at_offset<void>(geom, gl.records),
+        check(L.cgx_render_bwd_table((int)P, s.W, s.H, s.tanfovx, s.tanfovy, at_offset<uint32_t>(geom, gl.bins),
+                                     static_cast<uint32_t*>(list.data_ptr()), f32(bg), at_offset<void>(geom, gl.records),
                                      f32(out_map), at_offset<float>(img, il.accum_alpha),
                                      at_offset<uint32_t>(img, il.n_contrib), static_cast<uint8_t*>(local.data_ptr()),
                                      f32(d_color), f32(d_map), f32(d_depth), s.geo, f32(m2), f32(abs2), f32(co), f32(rgb),

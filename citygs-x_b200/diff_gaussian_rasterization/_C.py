@@ -270,11 +270,11 @@ _PREFETCH = _Prefetched()
 
 
 def prefetch_num_rendered(image_height, image_width, means2D, radii, compute_locally, depths=None):
-    """Launch the tile-count + prefix-sum stage of a coming render_gaussians call with these same tensors and let it
-    post the pair count (and, when `depths` is given, the depth range that lets the sort skip a pass) to pinned host
-    memory without waiting for it.  Not part of the reference's module."""
+    """Launch the counting stage of a coming render_gaussians call with these same tensors and let it post the pair
+    count to pinned host memory without waiting for it (`depths` is accepted and not needed).  Not part of the
+    reference's module."""
     if PROFILE is None:             # under profiling the render call counts for itself, between its own events
-        _lib.host().prefetch(int(image_height), int(image_width), means2D, radii, compute_locally, depths)
+        _lib.host().prefetch(int(image_height), int(image_width), means2D, radii, compute_locally)
 
 
 def _low_bits(dmin, dmax):
@@ -341,13 +341,12 @@ def render_gaussians(background, image_height, image_width, means2D, depths, rad
         imgBuffer = torch.empty(ilay.total(), dtype=torch.uint8, device=dev)
         im = ilay.views(imgBuffer)
         pre = _lib.host().take_prefetched(H, W, means2D, radii, local)
+        geomBuffer = torch.empty(glay.total(), dtype=torch.uint8, device=dev)
+        g = glay.views(geomBuffer)
+        _count_scan(l, P, W, H, radii, means2D, None if pre is not None else depths, local, g, st)
         if pre is not None:
-            geomBuffer, R, low_bits = pre
-            g = glay.views(geomBuffer)
+            R, low_bits = pre, 32
         else:
-            geomBuffer = torch.empty(glay.total(), dtype=torch.uint8, device=dev)
-            g = glay.views(geomBuffer)
-            _count_scan(l, P, W, H, radii, means2D, depths, local, g, st)
             # the key/value buffers are sized from the pair count: one host read, as in the reference
             R, dmin, dmax = g["num_rendered"][0:3].tolist()
             # depths of one view share their leading bits: the sort squeezes them out of its digits

@@ -121,7 +121,10 @@ SIGNATURES = {
     "cgx_bin_workspace_bytes": (_sz, [_i]),
     "cgx_bin_count_scan": (_i, [_i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "cgx_bin_count_scan_depths": (_i, [_i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
-    "cgx_bin_count_scan_post": (_i, [_i, _i, _i] + [_vp] * 7 + [_sz, _vp, _vp]),
+    "cgx_tile_bins_workspace_bytes": (_sz, [_i, _i]),
+    "cgx_tile_bins_longest": (_i, []),
+    "cgx_tile_bins_count": (_i, [_i, _i, _i] + [_vp] * 5 + [_sz, _vp, _vp]),
+    "cgx_tile_bins_sort": (_i, [_i, _i, _i] + [_vp] * 6 + [_sz, _vp, _vp, _vp]),
     "cgx_emit_keys": (_i, [_i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp]),
     "cgx_sort_workspace_bytes": (_sz, [_i64]),
     "cgx_sort_pairs": (_i, [_i64, _i, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
