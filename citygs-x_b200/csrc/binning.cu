@@ -766,53 +766,126 @@ tile_ranges_kernel(int64_t L, uint32_t T, const uint64_t* __restrict__ keys, uin
 // chip by (depth bits, Gaussian index), which is the order the stable sort of emitted keys leaves.  Four to six launches
 // instead of twenty, and 20 bytes per pair instead of 24 per pair and pass.
 
-constexpr int SMALL_TILE = 512, MID_TILE = 4096, LARGE_TILE = 16384;      // longest stretch of each kind of sorting CTA
+constexpr int KINDS = 4;                  // kinds of sorting CTA, by the longest stretch they take
+constexpr int KIND_0 = 512, KIND_1 = 2048, KIND_2 = 8192, KIND_3 = 16384;
 
 struct TileBins {
     uint2* ranges;            // (T)
-    uint32_t* counts;         // (T) pairs of the tile, then its next free place
+    uint32_t* counts;         // pairs of the tile, then its next free place, at counter(tile)
     MaskBand* band;
-    uint32_t* tiles;          // (3, T) tiles of each kind
-    uint32_t* n_tiles;        // (3) how many
+    uint32_t* tiles;          // (KINDS, T) tiles of each kind
+    uint32_t* n_tiles;        // (KINDS) how many
+    int eighth;               // T / 8, rounded up
+    // Atomics on one 32-byte sector of memory take turns, and the tiles with the longest lists lie side by side (a
+    // horizon): neighbours' counters are kept in different sectors.
+    __device__ __forceinline__ uint32_t* counter(int tile) const
+    {
+        return counts + (tile % eighth) * 8 + tile / eighth;
+    }
 };
 
 // One CTA: the mask as a band, and zeroed counts.
 __global__ void __launch_bounds__(1024)
 tile_bins_begin_kernel(int gx, int gy, const uint8_t* __restrict__ local, TileBins bins)
 {
-    for (int i = threadIdx.x; i < gx * gy; i += 1024) bins.counts[i] = 0;
-    if (threadIdx.x < 3) bins.n_tiles[threadIdx.x] = 0;
+    for (int i = threadIdx.x; i < 2 * bins.eighth; i += 1024)
+        reinterpret_cast<uint4*>(bins.counts)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x < KINDS) bins.n_tiles[threadIdx.x] = 0;
     analyse_mask(gx, gy, local, bins.band);
 }
 
-// Calls f(tile) for every local tile of the splat.
+// Calls f(owner lane, tile) for every local tile of the warp's 32 splats, a lane per (splat, tile) pair: the pairs are
+// numbered through, and a lane finds its pair's splat by a search over the running sums.  With a lane per splat the warp
+// took as many rounds as its widest splat has tiles (8-12 on aerial views with 23 pairs per warp, over 100 with large
+// splats), and each round's atomics had one or two lanes.  All 32 lanes call it.
 template <typename F>
-__device__ __forceinline__ void for_local_tiles(const float2 xy, int radius, const uint8_t* __restrict__ local, int gx,
-                                                int gy, const MaskBand band, F f)
+__device__ __forceinline__ void for_warp_tiles(const float2 xy, int radius, const uint8_t* __restrict__ local, int gx,
+                                               int gy, const MaskBand band, F f)
 {
-    uint2 lo, hi;
-    get_rect(xy, radius, lo, hi, gx, gy);
-    const int y0 = band.valid ? max((int)lo.y, band.row0) : (int)lo.y;
-    const int y1 = band.valid ? min((int)hi.y, band.row1) : (int)hi.y;
-    for (int y = y0; y < y1; y++)
-        for (int x = lo.x; x < (int)hi.x; x++)
-            if (band.valid || local[y * gx + x]) f(y * gx + x);
+    const int lane = threadIdx.x & 31;
+    int x0 = 0, y0 = 0, cols = 0, n = 0;
+    if (radius > 0) {
+        uint2 lo, hi;
+        get_rect(xy, radius, lo, hi, gx, gy);
+        x0 = lo.x;
+        y0 = band.valid ? max((int)lo.y, band.row0) : (int)lo.y;
+        const int y1 = band.valid ? min((int)hi.y, band.row1) : (int)hi.y;
+        cols = (int)hi.x - x0;
+        n = y1 > y0 && cols > 0 ? (y1 - y0) * cols : 0;
+    }
+    const int upto = (int)warp_incl_scan((uint32_t)n);
+    const int total = __shfl_sync(0xffffffffu, upto, 31);
+    for (int base = 0; base < total; base += 32) {
+        const int i = base + lane;
+        int owner = 0;                               // lanes whose pairs end at or before i
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+            if (__shfl_sync(0xffffffffu, upto, owner + step - 1) <= i) owner += step;
+        owner = min(owner, 31);
+        const int first = __shfl_sync(0xffffffffu, upto - n, owner), ox = __shfl_sync(0xffffffffu, x0, owner),
+                  oy = __shfl_sync(0xffffffffu, y0, owner), oc = __shfl_sync(0xffffffffu, cols, owner);
+        if (i < total) {
+            const int k = i - first, dy = k / oc, tile = (oy + dy) * gx + ox + (k - dy * oc);
+            if (band.valid || local[tile]) f(owner, tile);
+        }
+    }
 }
 
-__global__ void __launch_bounds__(CGX_BLOCK_SIZE)
-tile_bins_count_kernel(int P, int gx, int gy, const int* __restrict__ radii, const float2* __restrict__ means2D,
-                       const uint8_t* __restrict__ local, uint32_t* __restrict__ tiles_touched, const TileBins bins)
+// Four consecutive Gaussians per thread: one 128-bit load of radii tells whether anything else has to be read.
+constexpr int BIN_THREADS = 128, BIN_ITEMS = 4;
+struct FourSplats {
+    int4 r;
+    float2 xy[4];
+};
+__device__ __forceinline__ FourSplats load_four(int i, int P, const int* __restrict__ radii,
+                                                const float2* __restrict__ means2D, bool vec)
 {
-    const int i = blockIdx.x * CGX_BLOCK_SIZE + threadIdx.x;
-    if (i >= P) return;
-    const int r = radii[i];
-    uint32_t n = 0;
-    if (r > 0)
-        for_local_tiles(means2D[i], r, local, gx, gy, *bins.band, [&](int t) {
-            atomicAdd(&bins.counts[t], 1u);
-            n++;
-        });
-    tiles_touched[i] = n;
+    FourSplats s;
+    s.r = make_int4(0, 0, 0, 0);
+#pragma unroll
+    for (int k = 0; k < 4; k++) s.xy[k] = make_float2(0.f, 0.f);
+    if (vec && i + 4 <= P) {
+        s.r = *reinterpret_cast<const int4*>(radii + i);
+        if (s.r.x > 0 || s.r.y > 0 || s.r.z > 0 || s.r.w > 0) {
+            const float4 a = *reinterpret_cast<const float4*>(means2D + i), b = *reinterpret_cast<const float4*>(means2D + i + 2);
+            s.xy[0] = make_float2(a.x, a.y), s.xy[1] = make_float2(a.z, a.w);
+            s.xy[2] = make_float2(b.x, b.y), s.xy[3] = make_float2(b.z, b.w);
+        }
+    } else {
+        int* r = &s.r.x;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (i + k < P) {
+                r[k] = radii[i + k];
+                if (r[k] > 0) s.xy[k] = means2D[i + k];
+            }
+    }
+    return s;
+}
+
+__global__ void __launch_bounds__(BIN_THREADS)
+tile_bins_count_kernel(int P, int gx, int gy, const int* __restrict__ radii, const float2* __restrict__ means2D,
+                       const uint8_t* __restrict__ local, uint32_t* __restrict__ tiles_touched, const TileBins bins,
+                       const bool vec)
+{
+    const int i = (blockIdx.x * BIN_THREADS + threadIdx.x) * BIN_ITEMS;
+    const MaskBand band = *bins.band;
+    const FourSplats s = load_four(i, P, radii, means2D, vec);
+    const int r[4] = {s.r.x, s.r.y, s.r.z, s.r.w};
+    uint32_t n[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) n[k] = count_local_tiles(s.xy[k], r[k], local, gx, gy, band);
+    if (vec && i + 4 <= P) {
+        *reinterpret_cast<uint4*>(tiles_touched + i) = make_uint4(n[0], n[1], n[2], n[3]);
+    } else {
+        for (int k = 0; k < 4; k++)
+            if (i + k < P) tiles_touched[i + k] = n[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (__any_sync(0xffffffffu, n[k] != 0))
+            for_warp_tiles(s.xy[k], n[k] ? r[k] : 0, local, gx, gy, band,
+                           [&](int, int tile) { atomicAdd(bins.counter(tile), 1u); });
 }
 
 // One CTA: tile counts -> ranges and first free places, the lists of tiles by kind, and the words the host waits for:
@@ -821,22 +894,35 @@ tile_bins_count_kernel(int P, int gx, int gy, const int* __restrict__ radii, con
 __global__ void __launch_bounds__(1024)
 tile_bins_scan_kernel(int T, TileBins bins, volatile uint32_t* host_words)
 {
-    __shared__ uint32_t s_warp[32], s_max[32], s_kind[3];
+    __shared__ uint32_t s_warp[32], s_max[32], s_kind[KINDS];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    if (t < 3) s_kind[t] = 0;
+    if (t < KINDS) s_kind[t] = 0;
     uint32_t carry = 0, longest = 0;
     for (int start = 0; start < T; start += 8192) {
         uint32_t v[8], sum = 0;
+        unsigned long long kinds = 0;          // this thread's tiles of each kind, 16 bits each
         const int i0 = start + t * 8;
 #pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = i0 + k < T ? *bins.counter(i0 + k) : 0u;
+        auto kind_of = [](uint32_t n) { return n <= KIND_0 ? 0 : n <= KIND_1 ? 1 : n <= KIND_2 ? 2 : 3; };
+#pragma unroll
         for (int k = 0; k < 8; k++) {
-            v[k] = i0 + k < T ? bins.counts[i0 + k] : 0u;
             sum += v[k];
             longest = max(longest, v[k]);
+            if (v[k]) kinds += 1ull << (16 * kind_of(v[k]));
         }
         const uint32_t incl = warp_incl_scan(sum);
-        __syncthreads();                       // the previous round has read s_warp
+        unsigned long long kincl = kinds;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned long long up = __shfl_up_sync(0xffffffffu, kincl, d);
+            if (lane >= d) kincl += up;
+        }
+        const unsigned long long ktotal = __shfl_sync(0xffffffffu, kincl, 31);
+        __syncthreads();                       // the previous round has read s_warp; the counters are zero
         if (lane == 31) s_warp[warp] = incl;
+        uint32_t first = 0;
+        if (lane < KINDS) first = atomicAdd(&s_kind[lane], (uint32_t)(ktotal >> (16 * lane)) & 0xffffu);
         __syncthreads();
         uint32_t before = 0, total = 0;
 #pragma unroll
@@ -845,16 +931,20 @@ tile_bins_scan_kernel(int T, TileBins bins, volatile uint32_t* host_words)
             total += s_warp[w];
         }
         uint32_t at = carry + before + incl - sum;
+        uint32_t place[KINDS];
+#pragma unroll
+        for (int c = 0; c < KINDS; c++)
+            place[c] = __shfl_sync(0xffffffffu, first, c) + ((uint32_t)((kincl - kinds) >> (16 * c)) & 0xffffu);
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            if (i0 + k >= T) break;
-            bins.ranges[i0 + k] = make_uint2(at, at + v[k]);
-            bins.counts[i0 + k] = at;
-            at += v[k];
-            if (v[k]) {
-                const int kind = v[k] <= SMALL_TILE ? 0 : v[k] <= MID_TILE ? 1 : 2;
-                bins.tiles[(size_t)kind * T + atomicAdd(&s_kind[kind], 1u)] = i0 + k;
+            if (i0 + k < T) {
+                bins.ranges[i0 + k] = make_uint2(at, at + v[k]);
+                *bins.counter(i0 + k) = at;
             }
+            at += v[k];
+#pragma unroll
+            for (int c = 0; c < KINDS; c++)
+                if (v[k] && kind_of(v[k]) == c) bins.tiles[(size_t)c * T + place[c]++] = i0 + k;
         }
         carry += total;
     }
@@ -863,31 +953,48 @@ tile_bins_scan_kernel(int T, TileBins bins, volatile uint32_t* host_words)
     __syncthreads();
     if (t == 0) {
         for (int w = 1; w < 32; w++) longest = max(longest, s_max[w]);
-        for (int k = 0; k < 3; k++) bins.n_tiles[k] = s_kind[k];
+        for (int k = 0; k < KINDS; k++) bins.n_tiles[k] = s_kind[k];
         if (host_words) {
             host_words[0] = carry;
             host_words[1] = longest;
-            for (int k = 0; k < 3; k++) host_words[2 + k] = s_kind[k];
+            for (int k = 0; k < KINDS; k++) host_words[2 + k] = s_kind[k];
             __threadfence_system();
-            host_words[5] = 1u;
+            host_words[2 + KINDS] = 1u;
         }
     }
 }
 
-__global__ void __launch_bounds__(CGX_BLOCK_SIZE)
+__global__ void __launch_bounds__(BIN_THREADS)
 tile_bins_fill_kernel(int P, int gx, int gy, const int* __restrict__ radii, const float2* __restrict__ means2D,
                       const float* __restrict__ depths, const uint8_t* __restrict__ local, const TileBins bins,
-                      uint64_t* __restrict__ pairs, uint32_t capacity)
+                      uint64_t* __restrict__ pairs, uint32_t capacity, const bool vec)
 {
-    const int i = blockIdx.x * CGX_BLOCK_SIZE + threadIdx.x;
-    if (i >= P) return;
-    const int r = radii[i];
-    if (r <= 0) return;
-    const uint64_t pair = ((uint64_t)__float_as_uint(depths[i]) << 32) | (uint32_t)i;
-    for_local_tiles(means2D[i], r, local, gx, gy, *bins.band, [&](int t) {
-        const uint32_t at = atomicAdd(&bins.counts[t], 1u);
-        if (at < capacity) pairs[at] = pair;
-    });
+    // the owner's depth is fetched by index: a shuffle would need every lane, and not every lane has a pair
+    __shared__ uint32_t s_depth[4][BIN_THREADS];
+    const int i = (blockIdx.x * BIN_THREADS + threadIdx.x) * BIN_ITEMS;
+    const FourSplats s = load_four(i, P, radii, means2D, vec);
+    const int r[4] = {s.r.x, s.r.y, s.r.z, s.r.w};
+    const int warp0 = threadIdx.x & ~31;
+    const MaskBand band = *bins.band;
+    if (vec && i + 4 <= P) {
+        if (r[0] > 0 || r[1] > 0 || r[2] > 0 || r[3] > 0) {
+            const uint4 d = *reinterpret_cast<const uint4*>(depths + i);
+            s_depth[0][threadIdx.x] = d.x, s_depth[1][threadIdx.x] = d.y;
+            s_depth[2][threadIdx.x] = d.z, s_depth[3][threadIdx.x] = d.w;
+        }
+    } else {
+        for (int k = 0; k < 4; k++)
+            if (i + k < P) s_depth[k][threadIdx.x] = __float_as_uint(depths[i + k]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (__any_sync(0xffffffffu, r[k] > 0))
+            for_warp_tiles(s.xy[k], r[k], local, gx, gy, band, [&](int owner, int tile) {
+                const uint32_t id = (uint32_t)((blockIdx.x * BIN_THREADS + warp0 + owner) * BIN_ITEMS + k);
+                const uint32_t at = atomicAdd(bins.counter(tile), 1u);
+                if (at < capacity) pairs[at] = ((uint64_t)s_depth[k][warp0 + owner] << 32) | id;
+            });
 }
 
 // Sorts one tile's stretch per CTA: bucket sort by depth (as many buckets as there is room for pairs, spread over the
@@ -1770,10 +1877,11 @@ static size_t tile_bins_carve(int W, int H, void* workspace, TileBins* b)
     };
     TileBins t;
     t.ranges = (uint2*)take(T * sizeof(uint2));
-    t.counts = (uint32_t*)take(T * sizeof(uint32_t));
+    t.eighth = (int)((T + 7) / 8);
+    t.counts = (uint32_t*)take((size_t)t.eighth * 8 * sizeof(uint32_t));
     t.band = (MaskBand*)take(sizeof(MaskBand));
-    t.n_tiles = (uint32_t*)take(3 * sizeof(uint32_t));
-    t.tiles = (uint32_t*)take(3 * T * sizeof(uint32_t));
+    t.n_tiles = (uint32_t*)take(KINDS * sizeof(uint32_t));
+    t.tiles = (uint32_t*)take(KINDS * T * sizeof(uint32_t));
     if (b) *b = t;
     return at;
 }
@@ -1782,19 +1890,19 @@ extern "C" size_t cgx_tile_bins_workspace_bytes(int W, int H)
 {
     return W > 0 && H > 0 ? tile_bins_carve(W, H, nullptr, nullptr) : 0;
 }
-extern "C" int cgx_tile_bins_longest(void) { return LARGE_TILE; }
+extern "C" int cgx_tile_bins_longest(void) { return KIND_3; }
 
 extern "C" int cgx_tile_bins_count(int P, int W, int H, const int32_t* radii, const float* means2D,
                                    const uint8_t* compute_locally, uint32_t* tiles_touched, void* workspace,
-                                   size_t workspace_bytes, uint32_t* host_words6, void* stream)
+                                   size_t workspace_bytes, uint32_t* host_words7, void* stream)
 {
     if (P <= 0 || W <= 0 || H <= 0 || !radii || !means2D || ((uintptr_t)means2D & 7) || !compute_locally ||
         !tiles_touched || !workspace || ((uintptr_t)workspace & 7))
         return CGX_EINVAL;
     if (workspace_bytes < cgx_tile_bins_workspace_bytes(W, H)) return CGX_ENOMEM;
     void* mapped = nullptr;
-    if (host_words6) {       // fails for pageable memory: the caller must pass page-locked memory
-        cudaError_t e = cudaHostGetDevicePointer(&mapped, host_words6, 0);
+    if (host_words7) {       // fails for pageable memory: the caller must pass page-locked memory
+        cudaError_t e = cudaHostGetDevicePointer(&mapped, host_words7, 0);
         if (e != cudaSuccess || !mapped) { (void)cudaGetLastError(); return CGX_EINVAL; }
     }
     const int gx = (W + CGX_BLOCK_X - 1) / CGX_BLOCK_X, gy = (H + CGX_BLOCK_Y - 1) / CGX_BLOCK_Y;
@@ -1802,8 +1910,9 @@ extern "C" int cgx_tile_bins_count(int P, int W, int H, const int32_t* radii, co
     TileBins b;
     tile_bins_carve(W, H, workspace, &b);
     tile_bins_begin_kernel<<<1, 1024, 0, st>>>(gx, gy, compute_locally, b);
-    tile_bins_count_kernel<<<(P + CGX_BLOCK_SIZE - 1) / CGX_BLOCK_SIZE, CGX_BLOCK_SIZE, 0, st>>>(
-        P, gx, gy, radii, (const float2*)means2D, compute_locally, tiles_touched, b);
+    const bool vec = aligned16(radii) && aligned16(means2D) && aligned16(tiles_touched);
+    tile_bins_count_kernel<<<(P + BIN_THREADS * BIN_ITEMS - 1) / (BIN_THREADS * BIN_ITEMS), BIN_THREADS, 0, st>>>(
+        P, gx, gy, radii, (const float2*)means2D, compute_locally, tiles_touched, b, vec);
     tile_bins_scan_kernel<<<1, 1024, 0, st>>>(gx * gy, b, (volatile uint32_t*)mapped);
     return check_launch(3);
 }
@@ -1820,31 +1929,31 @@ static int launch_tile_sort(int n_tiles, const uint32_t* tiles, const uint2* ran
 }
 
 extern "C" int cgx_tile_bins_sort(int P, int W, int H, const int32_t* radii, const float* means2D, const float* depths,
-                                  const uint8_t* compute_locally, const uint32_t* host_words6, void* workspace,
+                                  const uint8_t* compute_locally, const uint32_t* host_words7, void* workspace,
                                   size_t workspace_bytes, uint64_t* pairs, uint32_t* point_list, void* stream)
 {
     if (P <= 0 || W <= 0 || H <= 0 || !radii || !means2D || ((uintptr_t)means2D & 7) || !depths || !compute_locally ||
-        !host_words6 || !workspace || ((uintptr_t)workspace & 7))
+        !host_words7 || !workspace || ((uintptr_t)workspace & 7))
         return CGX_EINVAL;
     if (workspace_bytes < cgx_tile_bins_workspace_bytes(W, H)) return CGX_ENOMEM;
-    const uint32_t R = host_words6[0];
+    const uint32_t R = host_words7[0];
     if (R == 0) return CGX_OK;
     if (!pairs || !point_list) return CGX_EINVAL;
-    if (host_words6[1] > (uint32_t)LARGE_TILE) return CGX_ENOMEM;
+    if (host_words7[1] > (uint32_t)KIND_3) return CGX_ENOMEM;
     const int gx = (W + CGX_BLOCK_X - 1) / CGX_BLOCK_X, gy = (H + CGX_BLOCK_Y - 1) / CGX_BLOCK_Y, T = gx * gy;
     cudaStream_t st = (cudaStream_t)stream;
     TileBins b;
     tile_bins_carve(W, H, workspace, &b);
-    tile_bins_fill_kernel<<<(P + CGX_BLOCK_SIZE - 1) / CGX_BLOCK_SIZE, CGX_BLOCK_SIZE, 0, st>>>(
-        P, gx, gy, radii, (const float2*)means2D, depths, compute_locally, b, pairs, R);
+    const bool vec = aligned16(radii) && aligned16(means2D) && aligned16(depths);
+    tile_bins_fill_kernel<<<(P + BIN_THREADS * BIN_ITEMS - 1) / (BIN_THREADS * BIN_ITEMS), BIN_THREADS, 0, st>>>(
+        P, gx, gy, radii, (const float2*)means2D, depths, compute_locally, b, pairs, R, vec);
     int s = check_launch();
     // long stretches first: their CTAs take longest
-    if (s == CGX_OK && host_words6[4])
-        s = launch_tile_sort<1024, LARGE_TILE>(host_words6[4], b.tiles + 2 * (size_t)T, b.ranges, pairs, point_list, st);
-    if (s == CGX_OK && host_words6[3])
-        s = launch_tile_sort<256, MID_TILE>(host_words6[3], b.tiles + T, b.ranges, pairs, point_list, st);
-    if (s == CGX_OK && host_words6[2])
-        s = launch_tile_sort<64, SMALL_TILE>(host_words6[2], b.tiles, b.ranges, pairs, point_list, st);
+    const uint32_t* n = host_words7 + 2;
+    if (s == CGX_OK && n[3]) s = launch_tile_sort<1024, KIND_3>(n[3], b.tiles + 3 * (size_t)T, b.ranges, pairs, point_list, st);
+    if (s == CGX_OK && n[2]) s = launch_tile_sort<512, KIND_2>(n[2], b.tiles + 2 * (size_t)T, b.ranges, pairs, point_list, st);
+    if (s == CGX_OK && n[1]) s = launch_tile_sort<256, KIND_1>(n[1], b.tiles + T, b.ranges, pairs, point_list, st);
+    if (s == CGX_OK && n[0]) s = launch_tile_sort<64, KIND_0>(n[0], b.tiles, b.ranges, pairs, point_list, st);
     return s;
 }
 

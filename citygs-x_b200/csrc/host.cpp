@@ -211,9 +211,9 @@ void report(const Stats& stats, const char* key, std::shared_ptr<EventMs> ms)
 // behind them that the host watches: neither a copy nor an event stands between the kernel and the launches that need them.
 constexpr int SLOTS = 256;
 struct Slot {
-    uint32_t word[5];          // see cgx_tile_bins_count
+    uint32_t word[6];          // see cgx_tile_bins_count
     volatile uint32_t flag;
-    uint32_t pad[2];
+    uint32_t pad;
 };
 Slot* slots()
 {
@@ -229,7 +229,7 @@ struct Count {
     Tensor geom;
     int slot = -1;
     cudaStream_t stream = nullptr;
-    uint32_t word[6];
+    uint32_t word[7];
     Tensor keep[3];            // a prefetched count's inputs: their addresses stay taken
 };
 std::mutex slot_lock;
@@ -281,7 +281,7 @@ void finish_count(Count& c)
         }
     }
     std::atomic_thread_fence(std::memory_order_acquire);
-    for (int k = 0; k < 5; k++) c.word[k] = s.word[k];
+    for (int k = 0; k < 6; k++) c.word[k] = s.word[k];
     give_slot(c.slot);
     c.slot = -1;
 }

@@ -1,5 +1,5 @@
 """The C++ operators (per-tile lists, C++ autograd nodes) against the Python nodes over the raw entry points (global
-sort), on lists around the lengths at which the per-tile sort changes its kind (512, 4096, 16384 and beyond), with
+sort), on lists around the lengths at which the per-tile sort changes its kind (512, 2048, 8192, 16384 and beyond), with
 depths spread, crowded and all equal, and with masks of every shape."""
 import pytest
 import torch
@@ -28,7 +28,7 @@ def run(t, cot, W, H, local, debug):
 
 
 @pytest.mark.parametrize("depths", ["spread", "crowded", "equal"])
-@pytest.mark.parametrize("P", [1, 63, 511, 512, 513, 4095, 4097, 16384, 20000])
+@pytest.mark.parametrize("P", [1, 63, 511, 512, 513, 2048, 2049, 8193, 16384, 20000])
 def test_lists_equal_the_global_sort(P, depths, cuda_device):
     t, cot, W, H = scene(P, 3.0, 0.02, cuda_device)
     if depths == "crowded":
