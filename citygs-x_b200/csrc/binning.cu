@@ -762,7 +762,7 @@ tile_ranges_kernel(int64_t L, uint32_t T, const uint64_t* __restrict__ keys, uin
 
 // ------------------------------------------------------------------------------------------------ lists per tile
 // The same lists without a global sort, for callers that need no sorted 64-bit keys: count the pairs of every tile,
-// scan the tiles, drop every pair (depth bits, Gaussian) into its tile's stretch in any order, and sort each stretch on
+// give every tile a stretch, drop every pair (depth bits, Gaussian) into its tile's stretch in any order, and sort each stretch on
 // chip by (depth bits, Gaussian index), which is the order the stable sort of emitted keys leaves.  Four to six launches
 // instead of twenty, and 20 bytes per pair instead of 24 per pair and pass.
 
@@ -775,6 +775,7 @@ struct TileBins {
     MaskBand* band;
     uint32_t* tiles;          // (KINDS, T) tiles of each kind
     uint32_t* n_tiles;        // (KINDS) how many
+    uint32_t* sums;           // pairs, longest stretch, CTAs that have scanned
     int eighth;               // T / 8, rounded up
     // Atomics on one 32-byte sector of memory take turns, and the tiles with the longest lists lie side by side (a
     // horizon): neighbours' counters are kept in different sectors.
@@ -791,44 +792,8 @@ tile_bins_begin_kernel(int gx, int gy, const uint8_t* __restrict__ local, TileBi
     for (int i = threadIdx.x; i < 2 * bins.eighth; i += 1024)
         reinterpret_cast<uint4*>(bins.counts)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (threadIdx.x < KINDS) bins.n_tiles[threadIdx.x] = 0;
+    if (threadIdx.x < 3) bins.sums[threadIdx.x] = 0;
     analyse_mask(gx, gy, local, bins.band);
-}
-
-// Calls f(owner lane, tile) for every local tile of the warp's 32 splats, a lane per (splat, tile) pair: the pairs are
-// numbered through, and a lane finds its pair's splat by a search over the running sums.  With a lane per splat the warp
-// took as many rounds as its widest splat has tiles (8-12 on aerial views with 23 pairs per warp, over 100 with large
-// splats), and each round's atomics had one or two lanes.  All 32 lanes call it.
-template <typename F>
-__device__ __forceinline__ void for_warp_tiles(const float2 xy, int radius, const uint8_t* __restrict__ local, int gx,
-                                               int gy, const MaskBand band, F f)
-{
-    const int lane = threadIdx.x & 31;
-    int x0 = 0, y0 = 0, cols = 0, n = 0;
-    if (radius > 0) {
-        uint2 lo, hi;
-        get_rect(xy, radius, lo, hi, gx, gy);
-        x0 = lo.x;
-        y0 = band.valid ? max((int)lo.y, band.row0) : (int)lo.y;
-        const int y1 = band.valid ? min((int)hi.y, band.row1) : (int)hi.y;
-        cols = (int)hi.x - x0;
-        n = y1 > y0 && cols > 0 ? (y1 - y0) * cols : 0;
-    }
-    const int upto = (int)warp_incl_scan((uint32_t)n);
-    const int total = __shfl_sync(0xffffffffu, upto, 31);
-    for (int base = 0; base < total; base += 32) {
-        const int i = base + lane;
-        int owner = 0;                               // lanes whose pairs end at or before i
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1)
-            if (__shfl_sync(0xffffffffu, upto, owner + step - 1) <= i) owner += step;
-        owner = min(owner, 31);
-        const int first = __shfl_sync(0xffffffffu, upto - n, owner), ox = __shfl_sync(0xffffffffu, x0, owner),
-                  oy = __shfl_sync(0xffffffffu, y0, owner), oc = __shfl_sync(0xffffffffu, cols, owner);
-        if (i < total) {
-            const int k = i - first, dy = k / oc, tile = (oy + dy) * gx + ox + (k - dy * oc);
-            if (band.valid || local[tile]) f(owner, tile);
-        }
-    }
 }
 
 // Four consecutive Gaussians per thread: one 128-bit load of radii tells whether anything else has to be read.
@@ -863,11 +828,70 @@ __device__ __forceinline__ FourSplats load_four(int i, int P, const int* __restr
     return s;
 }
 
+struct WarpRects {
+    uint4 first[32];            // per lane: number of the first pair of each of its four splats
+    uint32_t corner[4][32];     // x0 | y0 << 16
+    uint32_t cols[4][32];
+};
+
+// Calls f(owner lane, which of its four splats, tile) for every local tile of the warp's 128 splats, a lane per (splat,
+// tile) pair: the pairs are numbered through, and a lane finds its pair's splat by a search over the running sums.  With
+// a lane per splat the warp took as many rounds as its widest splat has tiles (8-12 on aerial views with 23 pairs per 32
+// splats, over 100 with large splats), and each round's atomics had one or two lanes.  All 32 lanes call it.
+template <typename F>
+__device__ __forceinline__ void for_warp_tiles(const FourSplats& s, const uint8_t* __restrict__ local, int gx, int gy,
+                                               const MaskBand band, WarpRects& rects, F f)
+{
+    const int lane = threadIdx.x & 31;
+    const int r[4] = {s.r.x, s.r.y, s.r.z, s.r.w};
+    uint32_t n[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        n[k] = 0;
+        if (r[k] > 0) {
+            uint2 lo, hi;
+            get_rect(s.xy[k], r[k], lo, hi, gx, gy);
+            const int y0 = band.valid ? max((int)lo.y, band.row0) : (int)lo.y;
+            const int y1 = band.valid ? min((int)hi.y, band.row1) : (int)hi.y;
+            const int cols = (int)hi.x - (int)lo.x;
+            if (y1 > y0 && cols > 0) {
+                n[k] = (y1 - y0) * cols;
+                rects.corner[k][lane] = lo.x | (uint32_t)y0 << 16;
+                rects.cols[k][lane] = cols;
+            }
+        }
+    }
+    const uint32_t mine = n[0] + n[1] + n[2] + n[3];
+    const uint32_t upto = warp_incl_scan(mine);
+    const uint32_t total = __shfl_sync(0xffffffffu, upto, 31), at = upto - mine;
+    if (total == 0) return;
+    rects.first[lane] = make_uint4(at, at + n[0], at + n[0] + n[1], at + n[0] + n[1] + n[2]);
+    __syncwarp();
+    for (uint32_t base = 0; base < total; base += 32) {
+        const uint32_t i = base + lane;
+        int owner = 0;                               // lanes whose pairs end at or before i
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+            if (__shfl_sync(0xffffffffu, upto, owner + step - 1) <= i) owner += step;
+        if (i < total) {
+            const uint4 first = rects.first[owner];
+            const int k = (i >= first.y) + (i >= first.z) + (i >= first.w);
+            const uint32_t j = i - (k == 0 ? first.x : k == 1 ? first.y : k == 2 ? first.z : first.w);
+            const uint32_t corner = rects.corner[k][owner], cols = rects.cols[k][owner], dy = j / cols;
+            const int tile = ((corner >> 16) + dy) * gx + (corner & 0xffffu) + (j - dy * cols);
+            if (band.valid || local[tile]) f(owner, k, tile);
+        }
+    }
+    __syncwarp();
+}
+
+// 20 M Gaussians, 4 % in view, 3840x2160: 87 us, 6 M at 1600x1200 (4.3 M pairs): 75 us.
 __global__ void __launch_bounds__(BIN_THREADS)
 tile_bins_count_kernel(int P, int gx, int gy, const int* __restrict__ radii, const float2* __restrict__ means2D,
                        const uint8_t* __restrict__ local, uint32_t* __restrict__ tiles_touched, const TileBins bins,
                        const bool vec)
 {
+    __shared__ WarpRects s_rects[BIN_THREADS / 32];
     const int i = (blockIdx.x * BIN_THREADS + threadIdx.x) * BIN_ITEMS;
     const MaskBand band = *bins.band;
     const FourSplats s = load_four(i, P, radii, means2D, vec);
@@ -881,125 +905,126 @@ tile_bins_count_kernel(int P, int gx, int gy, const int* __restrict__ radii, con
         for (int k = 0; k < 4; k++)
             if (i + k < P) tiles_touched[i + k] = n[k];
     }
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-        if (__any_sync(0xffffffffu, n[k] != 0))
-            for_warp_tiles(s.xy[k], n[k] ? r[k] : 0, local, gx, gy, band,
-                           [&](int, int tile) { atomicAdd(bins.counter(tile), 1u); });
+    if (__any_sync(0xffffffffu, (n[0] | n[1] | n[2] | n[3]) != 0))
+        for_warp_tiles(s, local, gx, gy, band, s_rects[threadIdx.x >> 5],
+                       [&](int, int, int tile) { atomicAdd(bins.counter(tile), 1u); });
 }
 
-// One CTA: tile counts -> ranges and first free places, the lists of tiles by kind, and the words the host waits for:
-// pairs, longest stretch, tiles of each kind, flag.  A thread takes eight consecutive tiles, so a 3840x2160 grid is four
-// rounds.
-__global__ void __launch_bounds__(1024)
+// Tile counts -> ranges and first free places, the lists of tiles by kind, and the words the host waits for: pairs,
+// longest stretch, tiles of each kind, flag.  The order of the stretches is of no account, so a CTA takes 2048 counters
+// as they lie in memory and its place by one atomic; the last CTA posts.
+__global__ void __launch_bounds__(256)
 tile_bins_scan_kernel(int T, TileBins bins, volatile uint32_t* host_words)
 {
-    __shared__ uint32_t s_warp[32], s_max[32], s_kind[KINDS];
+    __shared__ uint32_t s_warp[8], s_kind[KINDS], s_base, s_kind_base[KINDS];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     if (t < KINDS) s_kind[t] = 0;
-    uint32_t carry = 0, longest = 0;
-    for (int start = 0; start < T; start += 8192) {
-        uint32_t v[8], sum = 0;
-        unsigned long long kinds = 0;          // this thread's tiles of each kind, 16 bits each
-        const int i0 = start + t * 8;
+    const int sector = blockIdx.x * 256 + t;      // its eight counters are those of tiles sector + k * eighth
+    uint32_t v[8] = {0, 0, 0, 0, 0, 0, 0, 0}, sum = 0, longest = 0;
+    unsigned long long kinds = 0;                 // this thread's tiles of each kind, 16 bits each
+    auto kind_of = [](uint32_t n) { return n <= KIND_0 ? 0 : n <= KIND_1 ? 1 : n <= KIND_2 ? 2 : 3; };
+    if (sector < bins.eighth) {
+        const uint4* c = reinterpret_cast<const uint4*>(bins.counts) + 2 * sector;
+        const uint4 p = c[0], q = c[1];
+        v[0] = p.x, v[1] = p.y, v[2] = p.z, v[3] = p.w, v[4] = q.x, v[5] = q.y, v[6] = q.z, v[7] = q.w;
+    }
 #pragma unroll
-        for (int k = 0; k < 8; k++) v[k] = i0 + k < T ? *bins.counter(i0 + k) : 0u;
-        auto kind_of = [](uint32_t n) { return n <= KIND_0 ? 0 : n <= KIND_1 ? 1 : n <= KIND_2 ? 2 : 3; };
+    for (int k = 0; k < 8; k++) {
+        sum += v[k];
+        longest = max(longest, v[k]);
+        if (v[k]) kinds += 1ull << (16 * kind_of(v[k]));
+    }
+    const uint32_t incl = warp_incl_scan(sum);
+    unsigned long long kincl = kinds;
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            sum += v[k];
-            longest = max(longest, v[k]);
-            if (v[k]) kinds += 1ull << (16 * kind_of(v[k]));
-        }
-        const uint32_t incl = warp_incl_scan(sum);
-        unsigned long long kincl = kinds;
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned long long up = __shfl_up_sync(0xffffffffu, kincl, d);
+        if (lane >= d) kincl += up;
+    }
+    const unsigned long long ktotal = __shfl_sync(0xffffffffu, kincl, 31);
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t kfirst = 0;
+    if (lane < KINDS) kfirst = atomicAdd(&s_kind[lane], (uint32_t)(ktotal >> (16 * lane)) & 0xffffu);
+    if (lane == 0) atomicMax(&bins.sums[1], longest);
+    uint32_t before = 0, total = 0;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const unsigned long long up = __shfl_up_sync(0xffffffffu, kincl, d);
-            if (lane >= d) kincl += up;
-        }
-        const unsigned long long ktotal = __shfl_sync(0xffffffffu, kincl, 31);
-        __syncthreads();                       // the previous round has read s_warp; the counters are zero
-        if (lane == 31) s_warp[warp] = incl;
-        uint32_t first = 0;
-        if (lane < KINDS) first = atomicAdd(&s_kind[lane], (uint32_t)(ktotal >> (16 * lane)) & 0xffffu);
-        __syncthreads();
-        uint32_t before = 0, total = 0;
+    for (int w = 0; w < 8; w++) {
+        if (w < warp) before += s_warp[w];
+        total += s_warp[w];
+    }
+    __syncthreads();
+    if (t == 0) s_base = atomicAdd(&bins.sums[0], total);
+    else if (t >= 32 && t < 32 + KINDS) s_kind_base[t - 32] = atomicAdd(&bins.n_tiles[t - 32], s_kind[t - 32]);
+    __syncthreads();
+    uint32_t at = s_base + before + incl - sum, place[KINDS];
 #pragma unroll
-        for (int w = 0; w < 32; w++) {
-            if (w < warp) before += s_warp[w];
-            total += s_warp[w];
-        }
-        uint32_t at = carry + before + incl - sum;
-        uint32_t place[KINDS];
+    for (int c = 0; c < KINDS; c++)
+        place[c] = s_kind_base[c] + __shfl_sync(0xffffffffu, kfirst, c) + ((uint32_t)((kincl - kinds) >> (16 * c)) & 0xffffu);
+    uint32_t start[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int tile = k * bins.eighth + sector;
+        start[k] = at;
+        if (sector < bins.eighth && tile < T) bins.ranges[tile] = make_uint2(at, at + v[k]);
+        at += v[k];
 #pragma unroll
         for (int c = 0; c < KINDS; c++)
-            place[c] = __shfl_sync(0xffffffffu, first, c) + ((uint32_t)((kincl - kinds) >> (16 * c)) & 0xffffu);
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            if (i0 + k < T) {
-                bins.ranges[i0 + k] = make_uint2(at, at + v[k]);
-                *bins.counter(i0 + k) = at;
-            }
-            at += v[k];
-#pragma unroll
-            for (int c = 0; c < KINDS; c++)
-                if (v[k] && kind_of(v[k]) == c) bins.tiles[(size_t)c * T + place[c]++] = i0 + k;
-        }
-        carry += total;
+            if (v[k] && kind_of(v[k]) == c) bins.tiles[(size_t)c * T + place[c]++] = tile;
     }
-    longest = __reduce_max_sync(0xffffffffu, longest);
-    if (lane == 0) s_max[warp] = longest;
+    if (sector < bins.eighth) {
+        uint4* c = reinterpret_cast<uint4*>(bins.counts) + 2 * sector;
+        c[0] = make_uint4(start[0], start[1], start[2], start[3]);
+        c[1] = make_uint4(start[4], start[5], start[6], start[7]);
+    }
+    if (!host_words) return;
+    __threadfence();
     __syncthreads();
-    if (t == 0) {
-        for (int w = 1; w < 32; w++) longest = max(longest, s_max[w]);
-        for (int k = 0; k < KINDS; k++) bins.n_tiles[k] = s_kind[k];
-        if (host_words) {
-            host_words[0] = carry;
-            host_words[1] = longest;
-            for (int k = 0; k < KINDS; k++) host_words[2 + k] = s_kind[k];
-            __threadfence_system();
-            host_words[2 + KINDS] = 1u;
-        }
+    if (t == 0 && atomicAdd(&bins.sums[2], 1u) == gridDim.x - 1) {
+        __threadfence();
+        const volatile uint32_t *sums = bins.sums, *n_tiles = bins.n_tiles;
+        host_words[0] = sums[0];
+        host_words[1] = sums[1];
+        for (int k = 0; k < KINDS; k++) host_words[2 + k] = n_tiles[k];
+        __threadfence_system();
+        host_words[2 + KINDS] = 1u;
     }
 }
 
+// 75 us and 103 us for the two scenes above.
 __global__ void __launch_bounds__(BIN_THREADS)
 tile_bins_fill_kernel(int P, int gx, int gy, const int* __restrict__ radii, const float2* __restrict__ means2D,
                       const float* __restrict__ depths, const uint8_t* __restrict__ local, const TileBins bins,
                       uint64_t* __restrict__ pairs, uint32_t capacity, const bool vec)
 {
-    // the owner's depth is fetched by index: a shuffle would need every lane, and not every lane has a pair
+    __shared__ WarpRects s_rects[BIN_THREADS / 32];
     __shared__ uint32_t s_depth[4][BIN_THREADS];
     const int i = (blockIdx.x * BIN_THREADS + threadIdx.x) * BIN_ITEMS;
     const FourSplats s = load_four(i, P, radii, means2D, vec);
-    const int r[4] = {s.r.x, s.r.y, s.r.z, s.r.w};
+    const bool any = s.r.x > 0 || s.r.y > 0 || s.r.z > 0 || s.r.w > 0;
+    if (!__any_sync(0xffffffffu, any)) return;
     const int warp0 = threadIdx.x & ~31;
-    const MaskBand band = *bins.band;
-    if (vec && i + 4 <= P) {
-        if (r[0] > 0 || r[1] > 0 || r[2] > 0 || r[3] > 0) {
-            const uint4 d = *reinterpret_cast<const uint4*>(depths + i);
-            s_depth[0][threadIdx.x] = d.x, s_depth[1][threadIdx.x] = d.y;
-            s_depth[2][threadIdx.x] = d.z, s_depth[3][threadIdx.x] = d.w;
-        }
-    } else {
+    if (any && vec && i + 4 <= P) {
+        const uint4 d = *reinterpret_cast<const uint4*>(depths + i);
+        s_depth[0][threadIdx.x] = d.x, s_depth[1][threadIdx.x] = d.y;
+        s_depth[2][threadIdx.x] = d.z, s_depth[3][threadIdx.x] = d.w;
+    } else if (any) {
         for (int k = 0; k < 4; k++)
             if (i + k < P) s_depth[k][threadIdx.x] = __float_as_uint(depths[i + k]);
     }
     __syncwarp();
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-        if (__any_sync(0xffffffffu, r[k] > 0))
-            for_warp_tiles(s.xy[k], r[k], local, gx, gy, band, [&](int owner, int tile) {
-                const uint32_t id = (uint32_t)((blockIdx.x * BIN_THREADS + warp0 + owner) * BIN_ITEMS + k);
-                const uint32_t at = atomicAdd(bins.counter(tile), 1u);
-                if (at < capacity) pairs[at] = ((uint64_t)s_depth[k][warp0 + owner] << 32) | id;
-            });
+    for_warp_tiles(s, local, gx, gy, *bins.band, s_rects[threadIdx.x >> 5], [&](int owner, int k, int tile) {
+        const uint32_t id = (uint32_t)((blockIdx.x * BIN_THREADS + warp0 + owner) * BIN_ITEMS + k);
+        const uint32_t at = atomicAdd(bins.counter(tile), 1u);
+        if (at < capacity) pairs[at] = ((uint64_t)s_depth[k][warp0 + owner] << 32) | id;
+    });
 }
 
 // Sorts one tile's stretch per CTA: bucket sort by depth (as many buckets as there is room for pairs, spread over the
 // stretch's depth range), then every pair finds its place among the few of its bucket.  Where depths crowd into few
-// buckets that search would be quadratic: such a stretch is sorted by a bitonic network instead.
+// buckets that search would be quadratic: such a stretch is sorted by a bitonic network instead.  4.3 M pairs in 7500
+// tiles: 57 us for all kinds (the global sort of their emitted keys: 278 us); 8160 tiles of a 1920x1080 view: 12 us (84).
 constexpr uint32_t CROWDED = 96;      // pairs of one bucket from which the network is the cheaper way
 template <int THREADS, int MOST>
 __global__ void __launch_bounds__(THREADS)
@@ -1881,6 +1906,7 @@ static size_t tile_bins_carve(int W, int H, void* workspace, TileBins* b)
     t.counts = (uint32_t*)take((size_t)t.eighth * 8 * sizeof(uint32_t));
     t.band = (MaskBand*)take(sizeof(MaskBand));
     t.n_tiles = (uint32_t*)take(KINDS * sizeof(uint32_t));
+    t.sums = (uint32_t*)take(3 * sizeof(uint32_t));
     t.tiles = (uint32_t*)take(KINDS * T * sizeof(uint32_t));
     if (b) *b = t;
     return at;
@@ -1913,7 +1939,7 @@ extern "C" int cgx_tile_bins_count(int P, int W, int H, const int32_t* radii, co
     const bool vec = aligned16(radii) && aligned16(means2D) && aligned16(tiles_touched);
     tile_bins_count_kernel<<<(P + BIN_THREADS * BIN_ITEMS - 1) / (BIN_THREADS * BIN_ITEMS), BIN_THREADS, 0, st>>>(
         P, gx, gy, radii, (const float2*)means2D, compute_locally, tiles_touched, b, vec);
-    tile_bins_scan_kernel<<<1, 1024, 0, st>>>(gx * gy, b, (volatile uint32_t*)mapped);
+    tile_bins_scan_kernel<<<(b.eighth + 255) / 256, 256, 0, st>>>(gx * gy, b, (volatile uint32_t*)mapped);
     return check_launch(3);
 }
 

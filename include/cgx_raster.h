@@ -385,8 +385,8 @@ int cgx_bin_count_scan_depths(int P, int W, int H, const int32_t* radii, const f
                               const uint8_t* compute_locally, uint32_t* tiles_touched, uint32_t* num_rendered3,
                               void* workspace, size_t workspace_bytes, void* stream);
 
-/* Per-tile lists without sorted keys, for hosts that do not need those: the same point_list and ranges as emission,
- * sort and tile_ranges leave (each tile's Gaussians by depth bits, then index), in four to eight launches.
+/* Per-tile lists without sorted keys, for hosts that do not need those: for every tile the same list as emission, sort
+ * and tile_ranges leave (its Gaussians by depth bits, then index), the tiles' stretches in an order of their own, in four to eight launches.
  * cgx_tile_bins_count (P > 0) fills tiles_touched (P) and the workspace (8-byte aligned), whose first 2 T words are the
  * ranges, and posts seven words to page-locked host memory (optional): pairs, longest list, tiles of four kinds by list
  * length, and last a 1 that the caller clears before and watches after the call.  cgx_tile_bins_sort takes those words
