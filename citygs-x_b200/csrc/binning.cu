@@ -776,6 +776,7 @@ struct TileBins {
     uint32_t* tiles;          // (KINDS, T) tiles of each kind
     uint32_t* n_tiles;        // (KINDS) how many
     uint32_t* sums;           // pairs, longest stretch, CTAs that have scanned
+    uint32_t* before;         // (BIN_CTAS, 8 eighth) pairs of the tile in the CTAs that came before, at counter(tile)
     int eighth;               // T / 8, rounded up
     // Atomics on one 32-byte sector of memory take turns, and the tiles with the longest lists lie side by side (a
     // horizon): neighbours' counters are kept in different sectors.
@@ -908,6 +909,99 @@ tile_bins_count_kernel(int P, int gx, int gy, const int* __restrict__ radii, con
     if (__any_sync(0xffffffffu, (n[0] | n[1] | n[2] | n[3]) != 0))
         for_warp_tiles(s, local, gx, gy, band, s_rects[threadIdx.x >> 5],
                        [&](int, int, int tile) { atomicAdd(bins.counter(tile), 1u); });
+}
+
+// The two passes with the tiles' counters in shared memory, for Gaussians that outnumber the tiles: one CTA per SM takes
+// chunks of 128 Gaussians, and only its sums go to memory: the atomic returns what other CTAs have put there before, the
+// CTA's first place in the tile's stretch.  One atomic per CTA and tile instead of two per pair.  count + fill, us: 3.5 M
+// Gaussians in 391 tiles 900 -> 60 (64 sectors' worth of counters took all the atomics), 6 M in 7500 tiles 86 + 105 ->
+// 51 + 70, 1 M in 8160 tiles 12.5 + 13 -> 13 + 12; what is left is the numbering of the pairs (instructions).
+constexpr int BIN_CTAS = 148, BIN_WARPS = 32, BIN_CHUNK = 32 * BIN_ITEMS;
+constexpr int BIN_SHARED_TILES = 16384;           // 64 KB of counters next to 48 + 16 KB of the warps' rectangles, depths
+constexpr int BIN_SHARED_RATIO = 64;              // Gaussians per tile
+struct BinWarps {
+    WarpRects rects[BIN_WARPS];
+    uint32_t depth[BIN_WARPS][4][32];
+};
+
+__global__ void __launch_bounds__(32 * BIN_WARPS)
+tile_bins_count_shared_kernel(int P, int gx, int gy, const int* __restrict__ radii, const float2* __restrict__ means2D,
+                              const uint8_t* __restrict__ local, uint32_t* __restrict__ tiles_touched,
+                              const TileBins bins, const bool vec)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    WarpRects* s_rects = reinterpret_cast<WarpRects*>(smem_raw);
+    uint32_t* s_count = reinterpret_cast<uint32_t*>(s_rects + BIN_WARPS);        // 8 eighth: per tile
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slots = 8 * bins.eighth;
+    const MaskBand band = *bins.band;
+    for (int t = 4 * threadIdx.x; t < slots; t += 4 * 32 * BIN_WARPS)
+        *reinterpret_cast<uint4*>(s_count + t) = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    for (int64_t chunk = blockIdx.x + (int64_t)gridDim.x * warp; chunk * BIN_CHUNK < P; chunk += (int64_t)gridDim.x * BIN_WARPS) {
+        const int i = (int)chunk * BIN_CHUNK + lane * BIN_ITEMS;
+        const FourSplats s = load_four(i, P, radii, means2D, vec);
+        const int r[4] = {s.r.x, s.r.y, s.r.z, s.r.w};
+        uint32_t n[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) n[k] = count_local_tiles(s.xy[k], r[k], local, gx, gy, band);
+        if (vec && i + 4 <= P) {
+            *reinterpret_cast<uint4*>(tiles_touched + i) = make_uint4(n[0], n[1], n[2], n[3]);
+        } else {
+            for (int k = 0; k < 4; k++)
+                if (i + k < P) tiles_touched[i + k] = n[k];
+        }
+        if (__any_sync(0xffffffffu, (n[0] | n[1] | n[2] | n[3]) != 0))
+            for_warp_tiles(s, local, gx, gy, band, s_rects[warp], [&](int, int, int tile) { atomicAdd(s_count + tile, 1u); });
+    }
+    __syncthreads();
+    // every CTA starts elsewhere, and eight lanes share a sector
+    uint32_t* before = bins.before + (size_t)blockIdx.x * slots;
+    const int first = (int)((int64_t)blockIdx.x * slots / gridDim.x) & ~31;
+#pragma unroll 4
+    for (int j = threadIdx.x; j < slots; j += 32 * BIN_WARPS) {
+        const int at = j + first < slots ? j + first : j + first - slots;
+        const uint32_t v = s_count[(at & 7) * bins.eighth + (at >> 3)];
+        if (v) before[at] = atomicAdd(bins.counts + at, v);
+    }
+}
+
+__global__ void __launch_bounds__(32 * BIN_WARPS)
+tile_bins_fill_shared_kernel(int P, int gx, int gy, const int* __restrict__ radii, const float2* __restrict__ means2D,
+                             const float* __restrict__ depths, const uint8_t* __restrict__ local, const TileBins bins,
+                             uint64_t* __restrict__ pairs, uint32_t capacity, const bool vec)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    BinWarps& sw = *reinterpret_cast<BinWarps*>(smem_raw);
+    uint32_t* s_next = reinterpret_cast<uint32_t*>(&sw + 1);                     // 8 eighth: per tile
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slots = 8 * bins.eighth;
+    const MaskBand band = *bins.band;
+    // (a tile without pairs of this CTA gets a place that nothing uses)
+    const uint32_t* before = bins.before + (size_t)blockIdx.x * slots;
+#pragma unroll 4
+    for (int at = threadIdx.x; at < slots; at += 32 * BIN_WARPS)
+        s_next[(at & 7) * bins.eighth + (at >> 3)] = bins.counts[at] + before[at];
+    __syncthreads();
+    for (int64_t chunk = blockIdx.x + (int64_t)gridDim.x * warp; chunk * BIN_CHUNK < P; chunk += (int64_t)gridDim.x * BIN_WARPS) {
+        const int i = (int)chunk * BIN_CHUNK + lane * BIN_ITEMS;
+        const FourSplats s = load_four(i, P, radii, means2D, vec);
+        const bool any = s.r.x > 0 || s.r.y > 0 || s.r.z > 0 || s.r.w > 0;
+        if (!__any_sync(0xffffffffu, any)) continue;
+        uint32_t (&depth)[4][32] = sw.depth[warp];
+        if (any && vec && i + 4 <= P) {
+            const uint4 d = *reinterpret_cast<const uint4*>(depths + i);
+            depth[0][lane] = d.x, depth[1][lane] = d.y, depth[2][lane] = d.z, depth[3][lane] = d.w;
+        } else if (any) {
+            for (int k = 0; k < 4; k++)
+                if (i + k < P) depth[k][lane] = __float_as_uint(depths[i + k]);
+        }
+        __syncwarp();
+        for_warp_tiles(s, local, gx, gy, band, sw.rects[warp], [&](int owner, int k, int tile) {
+            const uint32_t id = (uint32_t)((int)chunk * BIN_CHUNK + owner * BIN_ITEMS + k);
+            const uint32_t at = atomicAdd(s_next + tile, 1u);
+            if (at < capacity) pairs[at] = ((uint64_t)depth[k][owner] << 32) | id;
+        });
+        __syncwarp();
+    }
 }
 
 // Tile counts -> ranges and first free places, the lists of tiles by kind, and the words the host waits for: pairs,
@@ -1908,9 +2002,15 @@ static size_t tile_bins_carve(int W, int H, void* workspace, TileBins* b)
     t.n_tiles = (uint32_t*)take(KINDS * sizeof(uint32_t));
     t.sums = (uint32_t*)take(3 * sizeof(uint32_t));
     t.tiles = (uint32_t*)take(KINDS * T * sizeof(uint32_t));
+    t.before = T <= BIN_SHARED_TILES ? (uint32_t*)take((size_t)BIN_CTAS * 8 * t.eighth * sizeof(uint32_t)) : nullptr;
     if (b) *b = t;
     return at;
 }
+
+// Counters in shared memory cost every CTA a pass over all tiles, whatever it has put there: at 32400 tiles 20 us of 45
+// against 31 with atomics per pair (3 M Gaussians), at 8160 tiles and 122 Gaussians per tile both take the same.
+static bool bins_in_shared(int P, int T) { return T <= BIN_SHARED_TILES && (int64_t)P >= (int64_t)BIN_SHARED_RATIO * T; }
+static int bins_shared_ctas(int P) { return (int)std::min<int64_t>(BIN_CTAS, ((int64_t)P + BIN_CHUNK - 1) / BIN_CHUNK); }
 
 extern "C" size_t cgx_tile_bins_workspace_bytes(int W, int H)
 {
@@ -1937,8 +2037,16 @@ extern "C" int cgx_tile_bins_count(int P, int W, int H, const int32_t* radii, co
     tile_bins_carve(W, H, workspace, &b);
     tile_bins_begin_kernel<<<1, 1024, 0, st>>>(gx, gy, compute_locally, b);
     const bool vec = aligned16(radii) && aligned16(means2D) && aligned16(tiles_touched);
-    tile_bins_count_kernel<<<(P + BIN_THREADS * BIN_ITEMS - 1) / (BIN_THREADS * BIN_ITEMS), BIN_THREADS, 0, st>>>(
-        P, gx, gy, radii, (const float2*)means2D, compute_locally, tiles_touched, b, vec);
+    if (bins_in_shared(P, gx * gy)) {
+        const int smem = BIN_WARPS * sizeof(WarpRects) + 8 * b.eighth * sizeof(uint32_t);
+        cudaError_t e = cudaFuncSetAttribute(tile_bins_count_shared_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) { set_cuda_error(e); return CGX_ECUDA; }
+        tile_bins_count_shared_kernel<<<bins_shared_ctas(P), 32 * BIN_WARPS, smem, st>>>(
+            P, gx, gy, radii, (const float2*)means2D, compute_locally, tiles_touched, b, vec);
+    } else {
+        tile_bins_count_kernel<<<(P + BIN_THREADS * BIN_ITEMS - 1) / (BIN_THREADS * BIN_ITEMS), BIN_THREADS, 0, st>>>(
+            P, gx, gy, radii, (const float2*)means2D, compute_locally, tiles_touched, b, vec);
+    }
     tile_bins_scan_kernel<<<(b.eighth + 255) / 256, 256, 0, st>>>(gx * gy, b, (volatile uint32_t*)mapped);
     return check_launch(3);
 }
@@ -1971,8 +2079,16 @@ extern "C" int cgx_tile_bins_sort(int P, int W, int H, const int32_t* radii, con
     TileBins b;
     tile_bins_carve(W, H, workspace, &b);
     const bool vec = aligned16(radii) && aligned16(means2D) && aligned16(depths);
-    tile_bins_fill_kernel<<<(P + BIN_THREADS * BIN_ITEMS - 1) / (BIN_THREADS * BIN_ITEMS), BIN_THREADS, 0, st>>>(
-        P, gx, gy, radii, (const float2*)means2D, depths, compute_locally, b, pairs, R, vec);
+    if (bins_in_shared(P, T)) {
+        const int smem = sizeof(BinWarps) + 8 * b.eighth * sizeof(uint32_t);
+        cudaError_t e = cudaFuncSetAttribute(tile_bins_fill_shared_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) { set_cuda_error(e); return CGX_ECUDA; }
+        tile_bins_fill_shared_kernel<<<bins_shared_ctas(P), 32 * BIN_WARPS, smem, st>>>(
+            P, gx, gy, radii, (const float2*)means2D, depths, compute_locally, b, pairs, R, vec);
+    } else {
+        tile_bins_fill_kernel<<<(P + BIN_THREADS * BIN_ITEMS - 1) / (BIN_THREADS * BIN_ITEMS), BIN_THREADS, 0, st>>>(
+            P, gx, gy, radii, (const float2*)means2D, depths, compute_locally, b, pairs, R, vec);
+    }
     int s = check_launch();
     // long stretches first: their CTAs take longest
     const uint32_t* n = host_words7 + 2;

@@ -82,3 +82,24 @@ def test_many_tiles_and_prefetch(cuda_device):
     for o in outs[1:]:
         for a, b in zip(o, outs[0]):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n,res", [(64 * 16384, (2048, 2048)), (64 * 16384 - 1, (2048, 2048)), (64 * 16512, (2064, 2048)),
+                                   (64 * 187 + 131, (265, 161)), (127, (16, 16)), (300_003, (129, 97))])
+def test_counters_in_either_memory(n, res, cuda_device):
+    """Gaussians and tiles around the sizes from which the tiles' counters lie in shared memory."""
+    from diff_gaussian_rasterization import GaussianRasterizer
+
+    g, cam = util.make_case(cfg=2, n=n, res=res)
+    dev = cuda_device
+    gd = {k: v.to(dev) for k, v in g.items()}
+    local = torch.ones((cam.H + 15) // 16, (cam.W + 15) // 16, dtype=torch.bool, device=dev)
+    outs = []
+    for debug in (True, False):
+        rast = GaussianRasterizer(util.settings_for(cam, dev, debug=debug))
+        m2, _, co, radii, depths = rast.preprocess_gaussians(gd["means3D"], gd["scales"], gd["rotations"], gd["sh"],
+                                                             gd["opacities"], util.cuda_args())
+        outs.append(rast.render_gaussians(m2, None, co, gd["rgb"], gd["all_map"], depths, radii, local, None,
+                                          util.cuda_args()))
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
