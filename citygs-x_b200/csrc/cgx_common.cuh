@@ -28,6 +28,36 @@ int post_words(const void* src_dev, void* dst_host_pinned, int n_words, cudaStre
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Two floats in one 64-bit register: sm_100a multiplies and adds such pairs with one instruction (each half rounded
+// as the scalar operation rounds it).
+struct Pair {
+    unsigned long long v;
+};
+__device__ __forceinline__ Pair pack(float a, float b)
+{
+    Pair p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(a), "f"(b));
+    return p;
+}
+__device__ __forceinline__ float2 unpack(const Pair p)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p.v));
+    return r;
+}
+__device__ __forceinline__ Pair fma2(const Pair a, const Pair b, const Pair c)
+{
+    Pair d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return d;
+}
+__device__ __forceinline__ Pair mul2(const Pair a, const Pair b)
+{
+    Pair d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+    return d;
+}
+
 __device__ __forceinline__ bool aligned16_dev(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Column-major 3x3 (m[c][r]); product order matches the usual column-major definition

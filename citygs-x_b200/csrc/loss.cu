@@ -49,36 +49,6 @@ __device__ __forceinline__ bool my_strip(Strip& st, int C, int H, int W, int seg
     return true;
 }
 
-// Two floats in one 64-bit register: sm_100a multiplies and adds such pairs with one instruction (each half rounded
-// as the scalar operation rounds it).
-struct Pair {
-    unsigned long long v;
-};
-__device__ __forceinline__ Pair pack(float a, float b)
-{
-    Pair p;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(a), "f"(b));
-    return p;
-}
-__device__ __forceinline__ float2 unpack(const Pair p)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p.v));
-    return r;
-}
-__device__ __forceinline__ Pair fma2(const Pair a, const Pair b, const Pair c)
-{
-    Pair d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return d;
-}
-__device__ __forceinline__ Pair mul2(const Pair a, const Pair b)
-{
-    Pair d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-    return d;
-}
-
 // Reads row y of N images into registers: columns x0 - 5 + lane, and for ten lanes x0 + 27 + lane; zero outside.
 template <int N>
 __device__ __forceinline__ void fetch_row(float (&v)[N][2], const float* const (&src)[N], int y, int x0, int H, int W,

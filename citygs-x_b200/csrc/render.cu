@@ -533,7 +533,7 @@ struct BwdOut {
 // of the dot products <features, cotangents>: one recurrence instead of eight.
 struct BwdPixel {
     float T, T_final_bg;                 // transmittance in front of the next contributor; T_final * <bg, dL/dC>
-    float last_alpha, last_dot, blend;
+    Pair behind[4];                      // the features blended behind the next contributor: r g | b m0 | m1 m2 | m3 m4
     float d[CGX_NCH + CGX_NMAP];         // cotangents: colour, plane map (with the plane depth's folded in)
 };
 
@@ -547,7 +547,8 @@ __device__ __forceinline__ void bwd_pixel_init(BwdPixel& px, bool inside, uint32
                                                const float* __restrict__ dL_dout_plane_depths, bool render_geo)
 {
     px.T = inside ? final_Ts[pix_id] : 0;
-    px.last_alpha = px.last_dot = px.blend = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) px.behind[k] = pack(0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < CGX_NCH + CGX_NMAP; i++) px.d[i] = 0.f;
     float bg_dot = 0.f;
@@ -580,7 +581,6 @@ __device__ __forceinline__ void bwd_pixel_init(BwdPixel& px, bool inside, uint32
 __device__ __forceinline__ float2 bwd_contribution(BwdPixel& px, const Record& r, const float opacity, const float G,
                                                    const float alpha)
 {
-    const float4 q2 = r.q2, q3 = r.q3;
     // one reciprocal serves both quotients: the hardware's approximation and a Newton step (within 0.51 ulp for these
     // arguments, 0.01 to 1, without the special cases that a general correctly rounded reciprocal carries along)
     const float one_ma = 1.f - alpha;
@@ -588,12 +588,20 @@ __device__ __forceinline__ float2 bwd_contribution(BwdPixel& px, const Record& r
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv_1ma) : "f"(one_ma));
     inv_1ma = fmaf(inv_1ma, fmaf(-one_ma, inv_1ma, 1.f), inv_1ma);
     px.T = px.T * inv_1ma;
-    const float dot = q2.x * px.d[0] + q2.y * px.d[1] + q2.z * px.d[2] + q2.w * px.d[3] + q3.x * px.d[4] +
-                      q3.y * px.d[5] + q3.z * px.d[6] + q3.w * px.d[7];
-    px.blend = px.last_alpha * px.last_dot + (1.f - px.last_alpha) * px.blend;
-    px.last_dot = dot;
-    px.last_alpha = alpha;
-    const float dL_dalpha = (dot - px.blend) * px.T - px.T_final_bg * inv_1ma;
+    // Channel by channel and in this order: behind the blended normal's projection on the ray the eight products cancel
+    // to four digits in places, and any other order of the same sum has other digits left there.
+    const ulonglong2 q2 = *reinterpret_cast<const ulonglong2*>(&r.q2), q3 = *reinterpret_cast<const ulonglong2*>(&r.q3);
+    const Pair feature[4] = {Pair{q2.x}, Pair{q2.y}, Pair{q3.x}, Pair{q3.y}};
+    const Pair minus_one = pack(-1.f, -1.f), alpha2 = pack(alpha, alpha), one_ma2 = pack(one_ma, one_ma);
+    float sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float2 ahead = unpack(fma2(px.behind[k], minus_one, feature[k]));
+        sum = fmaf(ahead.x, px.d[2 * k], sum);
+        sum = fmaf(ahead.y, px.d[2 * k + 1], sum);
+        px.behind[k] = fma2(alpha2, feature[k], mul2(one_ma2, px.behind[k]));
+    }
+    const float dL_dalpha = sum * px.T - px.T_final_bg * inv_1ma;
     return make_float2(alpha * px.T, opacity * G * dL_dalpha);
 }
 
