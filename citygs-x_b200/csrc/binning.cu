@@ -2039,8 +2039,8 @@ extern "C" int cgx_tile_bins_count(int P, int W, int H, const int32_t* radii, co
     const bool vec = aligned16(radii) && aligned16(means2D) && aligned16(tiles_touched);
     if (bins_in_shared(P, gx * gy)) {
         const int smem = BIN_WARPS * sizeof(WarpRects) + 8 * b.eighth * sizeof(uint32_t);
-        cudaError_t e = cudaFuncSetAttribute(tile_bins_count_shared_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) { set_cuda_error(e); return CGX_ECUDA; }
+        if (!allow_shared<tile_bins_count_shared_kernel>(BIN_WARPS * sizeof(WarpRects) + BIN_SHARED_TILES * sizeof(uint32_t)))
+            return CGX_ECUDA;
         tile_bins_count_shared_kernel<<<bins_shared_ctas(P), 32 * BIN_WARPS, smem, st>>>(
             P, gx, gy, radii, (const float2*)means2D, compute_locally, tiles_touched, b, vec);
     } else {
@@ -2056,8 +2056,7 @@ static int launch_tile_sort(int n_tiles, const uint32_t* tiles, const uint2* ran
                             uint32_t* list, cudaStream_t st)
 {
     constexpr int smem = MOST * sizeof(uint64_t) + MOST / 2 * sizeof(uint32_t);
-    cudaError_t e = cudaFuncSetAttribute(tile_sort_kernel<THREADS, MOST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) { set_cuda_error(e); return CGX_ECUDA; }
+    if (!allow_shared<tile_sort_kernel<THREADS, MOST>>(smem)) return CGX_ECUDA;
     tile_sort_kernel<THREADS, MOST><<<n_tiles, THREADS, smem, st>>>(tiles, ranges, pairs, list);
     return check_launch();
 }
@@ -2081,8 +2080,8 @@ extern "C" int cgx_tile_bins_sort(int P, int W, int H, const int32_t* radii, con
     const bool vec = aligned16(radii) && aligned16(means2D) && aligned16(depths);
     if (bins_in_shared(P, T)) {
         const int smem = sizeof(BinWarps) + 8 * b.eighth * sizeof(uint32_t);
-        cudaError_t e = cudaFuncSetAttribute(tile_bins_fill_shared_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) { set_cuda_error(e); return CGX_ECUDA; }
+        if (!allow_shared<tile_bins_fill_shared_kernel>(sizeof(BinWarps) + BIN_SHARED_TILES * sizeof(uint32_t)))
+            return CGX_ECUDA;
         tile_bins_fill_shared_kernel<<<bins_shared_ctas(P), 32 * BIN_WARPS, smem, st>>>(
             P, gx, gy, radii, (const float2*)means2D, depths, compute_locally, b, pairs, R, vec);
     } else {

@@ -6,6 +6,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
 #include "../../include/cgx_raster.h"
 #include "../../include/cgx_raster_testing.h"
 
@@ -56,6 +57,22 @@ __device__ __forceinline__ Pair mul2(const Pair a, const Pair b)
     Pair d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
     return d;
+}
+
+// Lets a kernel take more than 48 KB of dynamic shared memory; asked of the driver once per kernel and device (the call
+// takes a third of a microsecond, and a pass of a small scene made nine).
+template <auto KERNEL>
+inline bool allow_shared(int bytes)
+{
+    static std::atomic<bool> done[64];
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    const bool known = device >= 0 && device < 64;
+    if (e == cudaSuccess && known && done[device].load(std::memory_order_relaxed)) return true;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) { set_cuda_error(e); return false; }
+    if (known) done[device].store(true, std::memory_order_relaxed);
+    return true;
 }
 
 __device__ __forceinline__ bool aligned16_dev(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

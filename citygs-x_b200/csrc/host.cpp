@@ -8,6 +8,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <array>
 #include <atomic>
 #include <chrono>
 #include <map>
@@ -29,7 +30,7 @@ namespace {
     X(cgx_depth_normal_bwd) X(cgx_bin_workspace_bytes) X(cgx_bin_count_scan) X(cgx_emit_keys)                        \
     X(cgx_tile_bins_workspace_bytes) X(cgx_tile_bins_longest) X(cgx_tile_bins_count) X(cgx_tile_bins_sort)          \
     X(cgx_sort_workspace_bytes) X(cgx_sort_passes) X(cgx_sort_pairs_pingpong) X(cgx_tile_ranges) X(cgx_higher_msb)   \
-    X(cgx_render_records_bytes) X(cgx_render_fwd) X(cgx_render_bwd_workspace_bytes) X(cgx_render_bwd_table)
+    X(cgx_render_records_bytes) X(cgx_render_pack) X(cgx_render_fwd_packed) X(cgx_render_bwd_workspace_bytes) X(cgx_render_bwd_table)
 struct Library {
 #define X(f) decltype(&::f) f = nullptr;
     CGX_FUNCTIONS(X)
@@ -160,18 +161,49 @@ T* at_offset(const Tensor& buf, size_t off)
 
 // ---------------------------------------------------------------------------------------------- elapsed milliseconds
 // Resolved on first numeric use, so that the operators never block the host.
+constexpr int MOST_DEVICES = 64;
 struct EventMs {
     cudaEvent_t a = nullptr, b = nullptr;
     double ms = 0;
     bool have = false;
+    int device = 0;
+    // Pairs that a collector dropped are taken up again, as many as EVENTS_KEPT: creating and destroying one took 4 us.
+    struct Pool {
+        std::mutex lock;
+        std::vector<std::array<cudaEvent_t, 2>> pairs[MOST_DEVICES];
+    };
+    static constexpr size_t EVENTS_KEPT = 64;
+    static Pool& pool()
+    {
+        static Pool* p = new Pool;      // outlives every collector
+        return *p;
+    }
     EventMs()
     {
+        cudaGetDevice(&device);
+        if (device < MOST_DEVICES) {
+            Pool& p = pool();
+            std::lock_guard<std::mutex> g(p.lock);
+            if (!p.pairs[device].empty()) {
+                a = p.pairs[device].back()[0], b = p.pairs[device].back()[1];
+                p.pairs[device].pop_back();
+                return;
+            }
+        }
         cudaEventCreate(&a);
         cudaEventCreate(&b);
     }
     EventMs(const EventMs&) = delete;
     ~EventMs()
     {
+        if (device < MOST_DEVICES && a && b) {
+            Pool& p = pool();
+            std::lock_guard<std::mutex> g(p.lock);
+            if (p.pairs[device].size() < EVENTS_KEPT) {
+                p.pairs[device].push_back({a, b});
+                return;
+            }
+        }
         if (a) cudaEventDestroy(a);
         if (b) cudaEventDestroy(b);
     }
@@ -409,7 +441,8 @@ struct Render : torch::autograd::Function<Render> {
         Count count;
         if (!find_prefetched(count, means2D, radii, local, H, W))
             count = start_count(P, W, H, means2D, radii, local);
-        // allocated while the count is on its way
+        // allocated, and the records packed, while the count is on its way: it reaches the host about 8 us after the
+        // device has it, and the device would wait as long for the launches that need it
         const GeometryLayout gl(P, W, H);
         const ImageLayout il(HW);
         const Tensor n_render = empty_i32({T}, means2D), n_consider = empty_i32({T}, means2D),
@@ -417,6 +450,9 @@ struct Render : torch::autograd::Function<Render> {
                      color = empty_f32({3, H, W}, means2D), out_map = empty_f32({5, H, W}, means2D),
                      depth = empty_f32({1, H, W}, means2D), img = bytes_like(il.total, means2D);
         std::shared_ptr<EventMs> ms = stats ? std::make_shared<EventMs>() : nullptr;
+        if (ms) cudaEventRecord(ms->a, st);
+        check(L.cgx_render_pack((int)P, i32(radii), f32(means2D), f32(rgb), f32(all_map), f32(conic), s.geo,
+                                at_offset<void>(count.geom, gl.records), i32(observe), st), "cgx_render_pack");
         finish_count(count);
 
         const int64_t R = count.word[0];
@@ -425,7 +461,6 @@ struct Render : torch::autograd::Function<Render> {
         uint32_t* ranges = at_offset<uint32_t>(count.geom, gl.bins);
         uint8_t* loc = static_cast<uint8_t*>(local.data_ptr());
         uint32_t* ids = static_cast<uint32_t*>(list.data_ptr());
-        if (ms) cudaEventRecord(ms->a, st);
         if (count.word[1] <= (uint32_t)L.cgx_tile_bins_longest()) {
             const Tensor pairs = bytes_like(8 * R, means2D);
             check(L.cgx_tile_bins_sort((int)P, W, H, i32(radii), f32(means2D), f32(depths), loc, count.word,
@@ -434,7 +469,7 @@ struct Render : torch::autograd::Function<Render> {
         } else {
             sort_globally(P, R, W, H, T, radii, means2D, depths, loc, tiles, ids, ranges, st);
         }
-        check(L.cgx_render_fwd((int)P, W, H, s.tanfovx, s.tanfovy, ranges, ids, i32(radii), f32(means2D), f32(rgb),
+        check(L.cgx_render_fwd_packed((int)P, W, H, s.tanfovx, s.tanfovy, ranges, ids, i32(radii), f32(means2D), f32(rgb),
                                f32(all_map), f32(conic), loc, f32(bg), s.geo, at_offset<void>(count.geom, gl.records),
                                at_offset<float>(img, il.accum_alpha), at_offset<uint32_t>(img, il.n_contrib),
                                at_offset<uint32_t>(img, il.n_contrib2loss), f32(color), i32(observe), f32(out_map),

@@ -1413,9 +1413,7 @@ extern "C" int cgx_preprocess_bwd_batched_planes(int P, int B, const float* mean
     }
     const int vec_mask = (aligned16(means3D) ? 1 : 0) | (aligned16(scales) ? 2 : 0) | (aligned16(rotations) ? 4 : 0) |
                          (aligned16(dL_dmeans3D) ? 8 : 0) | (aligned16(dL_dscales) ? 16 : 0);
-    cudaError_t e = cudaFuncSetAttribute(preprocess_bwd_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sizeof(PreBwdSmem));
-    if (e != cudaSuccess) { set_cuda_error(e); return CGX_ECUDA; }
+    if (!allow_shared<preprocess_bwd_batched_kernel>((int)sizeof(PreBwdSmem))) return CGX_ECUDA;
     preprocess_bwd_batched_kernel<<<(P + CGX_BLOCK_SIZE - 1) / CGX_BLOCK_SIZE, CGX_BLOCK_SIZE, sizeof(PreBwdSmem),
                                     (cudaStream_t)stream>>>(P, means3D, scales, scale_modifier, rotations, cb, c, pl,
                                                             dL_dmeans3D, dL_dscales, (float4*)dL_drotations,

@@ -1056,7 +1056,7 @@ extern "C" int cgx_set_render_variant(int variant)
     return CGX_OK;
 }
 
-extern "C" int cgx_render_fwd(int P, int W, int H, float tanfovx, float tanfovy, const uint32_t* ranges,
+static int render_fwd(bool pack_first, int P, int W, int H, float tanfovx, float tanfovy, const uint32_t* ranges,
                               const uint32_t* point_list, const int32_t* radii, const float* means2D, const float* rgb, const float* all_map,
                               const float* conic_opacity, const uint8_t* compute_locally, const float* bg,
                               int render_geo, void* records, float* final_T, uint32_t* n_contrib,
@@ -1072,7 +1072,7 @@ extern "C" int cgx_render_fwd(int P, int W, int H, float tanfovx, float tanfovy,
         return CGX_EINVAL;
     if (P > 0 && (((uintptr_t)means2D & 7) || !aligned16(conic_opacity) || !aligned16(records))) return CGX_EINVAL;
     cudaStream_t st = (cudaStream_t)stream;
-    if (P > 0)
+    if (P > 0 && pack_first)
         pack_records_kernel<<<(P + 255) / 256, 256, 0, st>>>(P, radii, (const float2*)means2D,
                                                              (const float4*)conic_opacity, rgb, all_map, render_geo,
                                                              (Record*)records, out_observe);
@@ -1080,15 +1080,57 @@ extern "C" int cgx_render_fwd(int P, int W, int H, float tanfovx, float tanfovy,
     const float focal_x = W / (2.0f * tanfovx);
     const dim3 grid((W + CGX_BLOCK_X - 1) / CGX_BLOCK_X, (H + CGX_BLOCK_Y - 1) / CGX_BLOCK_Y, 1);
     const dim3 block(RENDER_THREADS, 1, 1);
-    auto kernel = (g_render_variant & 1) ? render_fwd_kernel<true> : render_fwd_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem));
-    if (e != cudaSuccess) { set_cuda_error(e); return CGX_ECUDA; }
+    const bool cull = g_render_variant & 1;
+    auto kernel = cull ? render_fwd_kernel<true> : render_fwd_kernel<false>;
+    if (!(cull ? allow_shared<render_fwd_kernel<true>>((int)sizeof(FwdSmem))
+               : allow_shared<render_fwd_kernel<false>>((int)sizeof(FwdSmem))))
+        return CGX_ECUDA;
     kernel<<<grid, block, sizeof(FwdSmem), st>>>(
         (const uint2*)ranges, point_list, W, H, focal_x, focal_y, float(W * 0.5f), float(H * 0.5f),
         (const Record*)records, final_T, n_contrib, n_contrib2loss, compute_locally, bg, out_color, out_observe,
         out_all_map, out_plane_depth, render_geo != 0, n_render_t, n_consider_t, n_contrib_t,
         P > 0 ? reinterpret_cast<unsigned long long*>((Record*)records + P) : nullptr);
-    return check_launch(P > 0 ? 2 : 1);
+    return check_launch(P > 0 && pack_first ? 2 : 1);
+}
+
+extern "C" int cgx_render_fwd(int P, int W, int H, float tanfovx, float tanfovy, const uint32_t* ranges,
+                              const uint32_t* point_list, const int32_t* radii, const float* means2D,
+                              const float* rgb, const float* all_map, const float* conic_opacity,
+                              const uint8_t* compute_locally, const float* bg, int render_geo, void* records,
+                              float* final_T, uint32_t* n_contrib, uint32_t* n_contrib2loss, float* out_color,
+                              int32_t* out_observe, float* out_all_map, float* out_plane_depth, int32_t* n_render_t,
+                              int32_t* n_consider_t, int32_t* n_contrib_t, void* stream)
+{
+    return render_fwd(true, P, W, H, tanfovx, tanfovy, ranges, point_list, radii, means2D, rgb, all_map, conic_opacity, compute_locally,
+                      bg, render_geo, records, final_T, n_contrib, n_contrib2loss, out_color, out_observe, out_all_map,
+                      out_plane_depth, n_render_t, n_consider_t, n_contrib_t, stream);
+}
+
+extern "C" int cgx_render_fwd_packed(int P, int W, int H, float tanfovx, float tanfovy, const uint32_t* ranges,
+                                     const uint32_t* point_list, const int32_t* radii, const float* means2D,
+                                     const float* rgb, const float* all_map, const float* conic_opacity,
+                                     const uint8_t* compute_locally, const float* bg, int render_geo, void* records,
+                                     float* final_T, uint32_t* n_contrib, uint32_t* n_contrib2loss, float* out_color,
+                                     int32_t* out_observe, float* out_all_map, float* out_plane_depth,
+                                     int32_t* n_render_t, int32_t* n_consider_t, int32_t* n_contrib_t, void* stream)
+{
+    return render_fwd(false, P, W, H, tanfovx, tanfovy, ranges, point_list, radii, means2D, rgb, all_map, conic_opacity, compute_locally,
+                      bg, render_geo, records, final_T, n_contrib, n_contrib2loss, out_color, out_observe, out_all_map,
+                      out_plane_depth, n_render_t, n_consider_t, n_contrib_t, stream);
+}
+
+extern "C" int cgx_render_pack(int P, const int32_t* radii, const float* means2D, const float* rgb, const float* all_map,
+                               const float* conic_opacity, int render_geo, void* records, int32_t* out_observe,
+                               void* stream)
+{
+    if (P < 0) return CGX_EINVAL;
+    if (P == 0) return CGX_OK;
+    if (!means2D || !rgb || !conic_opacity || !records || !out_observe || (render_geo && !all_map)) return CGX_EINVAL;
+    if (((uintptr_t)means2D & 7) || !aligned16(conic_opacity) || !aligned16(records)) return CGX_EINVAL;
+    pack_records_kernel<<<(P + 255) / 256, 256, 0, (cudaStream_t)stream>>>(P, radii, (const float2*)means2D,
+                                                                           (const float4*)conic_opacity, rgb, all_map,
+                                                                           render_geo, (Record*)records, out_observe);
+    return check_launch();
 }
 
 extern "C" int cgx_tile_stats(int W, int H, const uint32_t* ranges, const uint32_t* n_contrib_px,
@@ -1158,8 +1200,9 @@ extern "C" int cgx_render_bwd_table(int P, int W, int H, float tanfovx, float ta
         return check_launch(2);
     }
     auto kernel = table ? render_bwd_kernel<true> : render_bwd_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BwdSmem));
-    if (e != cudaSuccess) { set_cuda_error(e); return CGX_ECUDA; }
+    if (!(table ? allow_shared<render_bwd_kernel<true>>((int)sizeof(BwdSmem))
+                : allow_shared<render_bwd_kernel<false>>((int)sizeof(BwdSmem))))
+        return CGX_ECUDA;
     kernel<<<dim3(grid.x, grid.y * BWD_SPLIT), 32 * BWD_WARPS, sizeof(BwdSmem), st>>>(
         (const uint2*)ranges, point_list, W, H, focal_x, focal_y, bg, (const Record*)records, all_map_pixels, final_T,
         n_contrib, compute_locally, dL_dcolor, dL_dout_all_map, dL_dout_plane_depth, render_geo != 0, out, P,
@@ -1168,8 +1211,7 @@ extern "C" int cgx_render_bwd_table(int P, int W, int H, float tanfovx, float ta
         const int vec_ok = aligned16(dL_dmeans2D) && aligned16(dL_dmeans2D_abs) && aligned16(dL_dconic_opacity) &&
                            aligned16(dL_drgb) && aligned16(dL_dall_map);
         const int smem = 2 * sizeof(UnpackSlice);        // six CTAs per SM
-        e = cudaFuncSetAttribute(bwd_unpack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) { set_cuda_error(e); return CGX_ECUDA; }
+        if (!allow_shared<bwd_unpack_kernel>(smem)) return CGX_ECUDA;
         bwd_unpack_kernel<<<min((P + UNPACK_ROWS - 1) / UNPACK_ROWS, 148 * 6), UNPACK_ROWS, smem, st>>>(
             P, tiles_touched, out, render_geo != 0, vec_ok);
     }

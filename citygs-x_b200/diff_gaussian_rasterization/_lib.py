@@ -136,6 +136,8 @@ SIGNATURES = {
     "cgx_tile_ranges": (_i, [_i64, _i, _vp, _vp, _vp]),
     "cgx_render_records_bytes": (_sz, [_i]),
     "cgx_render_fwd": (_i, [_i, _i, _i, _f, _f] + [_vp] * 9 + [_i] + [_vp] * 12),
+    "cgx_render_fwd_packed": (_i, [_i, _i, _i, _f, _f] + [_vp] * 9 + [_i] + [_vp] * 12),
+    "cgx_render_pack": (_i, [_i] + [_vp] * 5 + [_i] + [_vp] * 3),
     "cgx_launch_count": (C.c_uint64, []),
     "cgx_tile_stats": (_i, [_i, _i] + [_vp] * 8),
     "cgx_render_bwd": (_i, [_i, _i, _i, _f, _f] + [_vp] * 11 + [_i] + [_vp] * 5 + [_i, _vp]),

@@ -475,6 +475,18 @@ int cgx_render_fwd(int P, int W, int H, float tanfovx, float tanfovy, const uint
                    float* out_color, int32_t* out_observe, float* out_all_map, float* out_plane_depth,
                    int32_t* n_render, int32_t* n_consider, int32_t* n_contrib_tile, void* stream);
 
+/* cgx_render_fwd in two calls, for hosts that have the records packed while they wait for the pair count:
+ * cgx_render_pack fills records and clears out_observe, cgx_render_fwd_packed does the rest (same arguments). */
+int cgx_render_pack(int P, const int32_t* radii /* optional */, const float* means2D, const float* rgb,
+                    const float* all_map, const float* conic_opacity, int render_geo, void* records,
+                    int32_t* out_observe, void* stream);
+int cgx_render_fwd_packed(int P, int W, int H, float tanfovx, float tanfovy, const uint32_t* ranges,
+                   const uint32_t* point_list, const int32_t* radii /* optional */, const float* means2D, const float* rgb, const float* all_map,
+                   const float* conic_opacity, const uint8_t* compute_locally, const float* bg, int render_geo,
+                   void* records, float* final_T, uint32_t* n_contrib, uint32_t* n_contrib2loss,
+                   float* out_color, int32_t* out_observe, float* out_all_map, float* out_plane_depth,
+                   int32_t* n_render, int32_t* n_consider, int32_t* n_contrib_tile, void* stream);
+
 /* get_n_render + reduce_data_per_block x2 (RAST/cuda_rasterizer/rasterizer_impl.cu:219-262,730-752):
  * per-tile int32 (T) outputs; every element written. */
 int cgx_tile_stats(int W, int H, const uint32_t* ranges, const uint32_t* n_contrib_px,
