@@ -918,7 +918,7 @@ tile_bins_count_kernel(int P, int gx, int gy, const int* __restrict__ radii, con
 // 51 + 70, 1 M in 8160 tiles 12.5 + 13 -> 13 + 12; what is left is the numbering of the pairs (instructions).
 constexpr int BIN_CTAS = 148, BIN_WARPS = 32, BIN_CHUNK = 32 * BIN_ITEMS;
 constexpr int BIN_SHARED_TILES = 16384;           // 64 KB of counters next to 48 + 16 KB of the warps' rectangles, depths
-constexpr int BIN_SHARED_RATIO = 64;              // Gaussians per tile
+constexpr int BIN_SHARED_RATIO = 32;              // Gaussians per tile
 struct BinWarps {
     WarpRects rects[BIN_WARPS];
     uint32_t depth[BIN_WARPS][4][32];
@@ -2008,7 +2008,8 @@ static size_t tile_bins_carve(int W, int H, void* workspace, TileBins* b)
 }
 
 // Counters in shared memory cost every CTA a pass over all tiles, whatever it has put there: at 32400 tiles 20 us of 45
-// against 31 with atomics per pair (3 M Gaussians), at 8160 tiles and 122 Gaussians per tile both take the same.
+// against 31 with atomics per pair (3 M Gaussians), at 8160 tiles and 122 Gaussians per tile both take the same, at 3600
+// tiles and 42 large splats per tile count + fill take 28 us of 42.
 static bool bins_in_shared(int P, int T) { return T <= BIN_SHARED_TILES && (int64_t)P >= (int64_t)BIN_SHARED_RATIO * T; }
 static int bins_shared_ctas(int P) { return (int)std::min<int64_t>(BIN_CTAS, ((int64_t)P + BIN_CHUNK - 1) / BIN_CHUNK); }
 

@@ -84,8 +84,8 @@ def test_many_tiles_and_prefetch(cuda_device):
             assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("n,res", [(64 * 16384, (2048, 2048)), (64 * 16384 - 1, (2048, 2048)), (64 * 16512, (2064, 2048)),
-                                   (64 * 187 + 131, (265, 161)), (127, (16, 16)), (300_003, (129, 97))])
+@pytest.mark.parametrize("n,res", [(32 * 16384, (2048, 2048)), (32 * 16384 - 1, (2048, 2048)), (32 * 16512, (2064, 2048)),
+                                   (32 * 187 + 131, (265, 161)), (127, (16, 16)), (300_003, (129, 97))])
 def test_counters_in_either_memory(n, res, cuda_device):
     """Gaussians and tiles around the sizes from which the tiles' counters lie in shared memory."""
     from diff_gaussian_rasterization import GaussianRasterizer
