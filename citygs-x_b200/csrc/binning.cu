@@ -7,6 +7,8 @@
 // (per-warp shared-memory counters filled with match.any ballots), again without inter-CTA spin waits:
 // per pass a histogram kernel, a 256-CTA digit-row scan and a scatter kernel that stages each CTA's
 // keys in shared memory so that every digit run leaves as a contiguous burst.
+#include <limits.h>
+#include <algorithm>
 #include "cgx_common.cuh"
 
 namespace cgx {
@@ -797,20 +799,25 @@ tile_bins_begin_kernel(int gx, int gy, const uint8_t* __restrict__ local, TileBi
     analyse_mask(gx, gy, local, bins.band);
 }
 
-// Four consecutive Gaussians per thread: one 128-bit load of radii tells whether anything else has to be read.
+// Four consecutive Gaussians per thread: one 128-bit load of radii tells whether anything else has to be read.  With
+// fewer Gaussians than would fill half of the warps that the chip holds this way, one per thread: 26 K splats of 40 tiles
+// each in a 3078x2031 view count + fill 169 -> 60 us, 150 K large ones at 1280x720 28 -> 22.
 constexpr int BIN_THREADS = 128, BIN_ITEMS = 4;
 struct FourSplats {
     int4 r;
     float2 xy[4];
 };
-__device__ __forceinline__ FourSplats load_four(int i, int P, const int* __restrict__ radii,
-                                                const float2* __restrict__ means2D, bool vec)
+__device__ __forceinline__ FourSplats load_splats(int i, int P, int items, const int* __restrict__ radii,
+                                                  const float2* __restrict__ means2D, bool vec)
 {
     FourSplats s;
     s.r = make_int4(0, 0, 0, 0);
 #pragma unroll
     for (int k = 0; k < 4; k++) s.xy[k] = make_float2(0.f, 0.f);
-    if (vec && i + 4 <= P) {
+    if (items == 1) {
+        if (i < P) s.r.x = radii[i];
+        if (s.r.x > 0) s.xy[0] = means2D[i];
+    } else if (vec && i + 4 <= P) {
         s.r = *reinterpret_cast<const int4*>(radii + i);
         if (s.r.x > 0 || s.r.y > 0 || s.r.z > 0 || s.r.w > 0) {
             const float4 a = *reinterpret_cast<const float4*>(means2D + i), b = *reinterpret_cast<const float4*>(means2D + i + 2);
@@ -890,17 +897,19 @@ __device__ __forceinline__ void for_warp_tiles(const FourSplats& s, const uint8_
 __global__ void __launch_bounds__(BIN_THREADS)
 tile_bins_count_kernel(int P, int gx, int gy, const int* __restrict__ radii, const float2* __restrict__ means2D,
                        const uint8_t* __restrict__ local, uint32_t* __restrict__ tiles_touched, const TileBins bins,
-                       const bool vec)
+                       const bool vec, const int items)
 {
     __shared__ WarpRects s_rects[BIN_THREADS / 32];
-    const int i = (blockIdx.x * BIN_THREADS + threadIdx.x) * BIN_ITEMS;
+    const int i = (blockIdx.x * BIN_THREADS + threadIdx.x) * items;
     const MaskBand band = *bins.band;
-    const FourSplats s = load_four(i, P, radii, means2D, vec);
+    const FourSplats s = load_splats(i, P, items, radii, means2D, vec);
     const int r[4] = {s.r.x, s.r.y, s.r.z, s.r.w};
     uint32_t n[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) n[k] = count_local_tiles(s.xy[k], r[k], local, gx, gy, band);
-    if (vec && i + 4 <= P) {
+    if (items == 1) {
+        if (i < P) tiles_touched[i] = n[0];
+    } else if (vec && i + 4 <= P) {
         *reinterpret_cast<uint4*>(tiles_touched + i) = make_uint4(n[0], n[1], n[2], n[3]);
     } else {
         for (int k = 0; k < 4; k++)
@@ -912,7 +921,7 @@ tile_bins_count_kernel(int P, int gx, int gy, const int* __restrict__ radii, con
 }
 
 // The two passes with the tiles' counters in shared memory, for Gaussians that outnumber the tiles: one CTA per SM takes
-// chunks of 128 Gaussians, and only its sums go to memory: the atomic returns what other CTAs have put there before, the
+// chunks of 128 (or 32) Gaussians, and only its sums go to memory: the atomic returns what other CTAs have put there before, the
 // CTA's first place in the tile's stretch.  One atomic per CTA and tile instead of two per pair.  count + fill, us: 3.5 M
 // Gaussians in 391 tiles 900 -> 60 (64 sectors' worth of counters took all the atomics), 6 M in 7500 tiles 86 + 105 ->
 // 51 + 70, 1 M in 8160 tiles 12.5 + 13 -> 13 + 12; what is left is the numbering of the pairs (instructions).
@@ -927,24 +936,27 @@ struct BinWarps {
 __global__ void __launch_bounds__(32 * BIN_WARPS)
 tile_bins_count_shared_kernel(int P, int gx, int gy, const int* __restrict__ radii, const float2* __restrict__ means2D,
                               const uint8_t* __restrict__ local, uint32_t* __restrict__ tiles_touched,
-                              const TileBins bins, const bool vec)
+                              const TileBins bins, const bool vec, const int items)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WarpRects* s_rects = reinterpret_cast<WarpRects*>(smem_raw);
     uint32_t* s_count = reinterpret_cast<uint32_t*>(s_rects + BIN_WARPS);        // 8 eighth: per tile
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slots = 8 * bins.eighth;
+    const int chunk_size = 32 * items;
     const MaskBand band = *bins.band;
     for (int t = 4 * threadIdx.x; t < slots; t += 4 * 32 * BIN_WARPS)
         *reinterpret_cast<uint4*>(s_count + t) = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
-    for (int64_t chunk = blockIdx.x + (int64_t)gridDim.x * warp; chunk * BIN_CHUNK < P; chunk += (int64_t)gridDim.x * BIN_WARPS) {
-        const int i = (int)chunk * BIN_CHUNK + lane * BIN_ITEMS;
-        const FourSplats s = load_four(i, P, radii, means2D, vec);
+    for (int64_t chunk = blockIdx.x + (int64_t)gridDim.x * warp; chunk * chunk_size < P; chunk += (int64_t)gridDim.x * BIN_WARPS) {
+        const int i = (int)chunk * chunk_size + lane * items;
+        const FourSplats s = load_splats(i, P, items, radii, means2D, vec);
         const int r[4] = {s.r.x, s.r.y, s.r.z, s.r.w};
         uint32_t n[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) n[k] = count_local_tiles(s.xy[k], r[k], local, gx, gy, band);
-        if (vec && i + 4 <= P) {
+        if (items == 1) {
+            if (i < P) tiles_touched[i] = n[0];
+        } else if (vec && i + 4 <= P) {
             *reinterpret_cast<uint4*>(tiles_touched + i) = make_uint4(n[0], n[1], n[2], n[3]);
         } else {
             for (int k = 0; k < 4; k++)
@@ -968,12 +980,13 @@ tile_bins_count_shared_kernel(int P, int gx, int gy, const int* __restrict__ rad
 __global__ void __launch_bounds__(32 * BIN_WARPS)
 tile_bins_fill_shared_kernel(int P, int gx, int gy, const int* __restrict__ radii, const float2* __restrict__ means2D,
                              const float* __restrict__ depths, const uint8_t* __restrict__ local, const TileBins bins,
-                             uint64_t* __restrict__ pairs, uint32_t capacity, const bool vec)
+                             uint64_t* __restrict__ pairs, uint32_t capacity, const bool vec, const int items)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BinWarps& sw = *reinterpret_cast<BinWarps*>(smem_raw);
     uint32_t* s_next = reinterpret_cast<uint32_t*>(&sw + 1);                     // 8 eighth: per tile
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slots = 8 * bins.eighth;
+    const int chunk_size = 32 * items;
     const MaskBand band = *bins.band;
     // (a tile without pairs of this CTA gets a place that nothing uses)
     const uint32_t* before = bins.before + (size_t)blockIdx.x * slots;
@@ -981,13 +994,15 @@ tile_bins_fill_shared_kernel(int P, int gx, int gy, const int* __restrict__ radi
     for (int at = threadIdx.x; at < slots; at += 32 * BIN_WARPS)
         s_next[(at & 7) * bins.eighth + (at >> 3)] = bins.counts[at] + before[at];
     __syncthreads();
-    for (int64_t chunk = blockIdx.x + (int64_t)gridDim.x * warp; chunk * BIN_CHUNK < P; chunk += (int64_t)gridDim.x * BIN_WARPS) {
-        const int i = (int)chunk * BIN_CHUNK + lane * BIN_ITEMS;
-        const FourSplats s = load_four(i, P, radii, means2D, vec);
+    for (int64_t chunk = blockIdx.x + (int64_t)gridDim.x * warp; chunk * chunk_size < P; chunk += (int64_t)gridDim.x * BIN_WARPS) {
+        const int i = (int)chunk * chunk_size + lane * items;
+        const FourSplats s = load_splats(i, P, items, radii, means2D, vec);
         const bool any = s.r.x > 0 || s.r.y > 0 || s.r.z > 0 || s.r.w > 0;
         if (!__any_sync(0xffffffffu, any)) continue;
         uint32_t (&depth)[4][32] = sw.depth[warp];
-        if (any && vec && i + 4 <= P) {
+        if (items == 1) {
+            if (any) depth[0][lane] = __float_as_uint(depths[i]);
+        } else if (any && vec && i + 4 <= P) {
             const uint4 d = *reinterpret_cast<const uint4*>(depths + i);
             depth[0][lane] = d.x, depth[1][lane] = d.y, depth[2][lane] = d.z, depth[3][lane] = d.w;
         } else if (any) {
@@ -996,7 +1011,7 @@ tile_bins_fill_shared_kernel(int P, int gx, int gy, const int* __restrict__ radi
         }
         __syncwarp();
         for_warp_tiles(s, local, gx, gy, band, sw.rects[warp], [&](int owner, int k, int tile) {
-            const uint32_t id = (uint32_t)((int)chunk * BIN_CHUNK + owner * BIN_ITEMS + k);
+            const uint32_t id = (uint32_t)((int)chunk * chunk_size + owner * items + k);
             const uint32_t at = atomicAdd(s_next + tile, 1u);
             if (at < capacity) pairs[at] = ((uint64_t)depth[k][owner] << 32) | id;
         });
@@ -1005,10 +1020,10 @@ tile_bins_fill_shared_kernel(int P, int gx, int gy, const int* __restrict__ radi
 }
 
 // Tile counts -> ranges and first free places, the lists of tiles by kind, and the words the host waits for: pairs,
-// longest stretch, tiles of each kind, flag.  The order of the stretches is of no account, so a CTA takes 2048 counters
-// as they lie in memory and its place by one atomic; the last CTA posts.
+// longest stretch, tiles of each kind.  The order of the stretches is of no account, so a CTA takes 2048 counters
+// as they lie in memory and its place by one atomic; the last CTA posts, before it writes what only the device reads.
 __global__ void __launch_bounds__(256)
-tile_bins_scan_kernel(int T, TileBins bins, volatile uint32_t* host_words)
+tile_bins_scan_kernel(int T, TileBins bins, volatile unsigned long long* host_words)
 {
     __shared__ uint32_t s_warp[8], s_kind[KINDS], s_base, s_kind_base[KINDS];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -1052,6 +1067,16 @@ tile_bins_scan_kernel(int T, TileBins bins, volatile uint32_t* host_words)
     if (t == 0) s_base = atomicAdd(&bins.sums[0], total);
     else if (t >= 32 && t < 32 + KINDS) s_kind_base[t - 32] = atomicAdd(&bins.n_tiles[t - 32], s_kind[t - 32]);
     __syncthreads();
+    if (t == 0 && host_words) {       // (the barrier puts this CTA's sums before the fence)
+        __threadfence();
+        if (atomicAdd(&bins.sums[2], 1u) == gridDim.x - 1) {
+            __threadfence();
+            const volatile uint32_t *sums = bins.sums, *n_tiles = bins.n_tiles;
+            const uint32_t word[2 + KINDS] = {sums[0], sums[1], n_tiles[0], n_tiles[1], n_tiles[2], n_tiles[3]};
+            // each word with a flag of its own: nothing has to be ordered, which took 2 us
+            for (int k = 0; k < 2 + KINDS; k++) host_words[k] = 1ull << 32 | word[k];
+        }
+    }
     uint32_t at = s_base + before + incl - sum, place[KINDS];
 #pragma unroll
     for (int c = 0; c < KINDS; c++)
@@ -1072,34 +1097,24 @@ tile_bins_scan_kernel(int T, TileBins bins, volatile uint32_t* host_words)
         c[0] = make_uint4(start[0], start[1], start[2], start[3]);
         c[1] = make_uint4(start[4], start[5], start[6], start[7]);
     }
-    if (!host_words) return;
-    __threadfence();
-    __syncthreads();
-    if (t == 0 && atomicAdd(&bins.sums[2], 1u) == gridDim.x - 1) {
-        __threadfence();
-        const volatile uint32_t *sums = bins.sums, *n_tiles = bins.n_tiles;
-        host_words[0] = sums[0];
-        host_words[1] = sums[1];
-        for (int k = 0; k < KINDS; k++) host_words[2 + k] = n_tiles[k];
-        __threadfence_system();
-        host_words[2 + KINDS] = 1u;
-    }
 }
 
 // 75 us and 103 us for the two scenes above.
 __global__ void __launch_bounds__(BIN_THREADS)
 tile_bins_fill_kernel(int P, int gx, int gy, const int* __restrict__ radii, const float2* __restrict__ means2D,
                       const float* __restrict__ depths, const uint8_t* __restrict__ local, const TileBins bins,
-                      uint64_t* __restrict__ pairs, uint32_t capacity, const bool vec)
+                      uint64_t* __restrict__ pairs, uint32_t capacity, const bool vec, const int items)
 {
     __shared__ WarpRects s_rects[BIN_THREADS / 32];
     __shared__ uint32_t s_depth[4][BIN_THREADS];
-    const int i = (blockIdx.x * BIN_THREADS + threadIdx.x) * BIN_ITEMS;
-    const FourSplats s = load_four(i, P, radii, means2D, vec);
+    const int i = (blockIdx.x * BIN_THREADS + threadIdx.x) * items;
+    const FourSplats s = load_splats(i, P, items, radii, means2D, vec);
     const bool any = s.r.x > 0 || s.r.y > 0 || s.r.z > 0 || s.r.w > 0;
     if (!__any_sync(0xffffffffu, any)) return;
     const int warp0 = threadIdx.x & ~31;
-    if (any && vec && i + 4 <= P) {
+    if (items == 1) {
+        if (any) s_depth[0][threadIdx.x] = __float_as_uint(depths[i]);
+    } else if (any && vec && i + 4 <= P) {
         const uint4 d = *reinterpret_cast<const uint4*>(depths + i);
         s_depth[0][threadIdx.x] = d.x, s_depth[1][threadIdx.x] = d.y;
         s_depth[2][threadIdx.x] = d.z, s_depth[3][threadIdx.x] = d.w;
@@ -1109,7 +1124,7 @@ tile_bins_fill_kernel(int P, int gx, int gy, const int* __restrict__ radii, cons
     }
     __syncwarp();
     for_warp_tiles(s, local, gx, gy, *bins.band, s_rects[threadIdx.x >> 5], [&](int owner, int k, int tile) {
-        const uint32_t id = (uint32_t)((blockIdx.x * BIN_THREADS + warp0 + owner) * BIN_ITEMS + k);
+        const uint32_t id = (uint32_t)((blockIdx.x * BIN_THREADS + warp0 + owner) * items + k);
         const uint32_t at = atomicAdd(bins.counter(tile), 1u);
         if (at < capacity) pairs[at] = ((uint64_t)s_depth[k][warp0 + owner] << 32) | id;
     });
@@ -2011,7 +2026,12 @@ static size_t tile_bins_carve(int W, int H, void* workspace, TileBins* b)
 // against 31 with atomics per pair (3 M Gaussians), at 8160 tiles and 122 Gaussians per tile both take the same, at 3600
 // tiles and 42 large splats per tile count + fill take 28 us of 42.
 static bool bins_in_shared(int P, int T) { return T <= BIN_SHARED_TILES && (int64_t)P >= (int64_t)BIN_SHARED_RATIO * T; }
-static int bins_shared_ctas(int P) { return (int)std::min<int64_t>(BIN_CTAS, ((int64_t)P + BIN_CHUNK - 1) / BIN_CHUNK); }
+static int bins_items(int P) { return P <= BIN_CTAS * BIN_WARPS * BIN_CHUNK / 2 ? 1 : BIN_ITEMS; }
+static int bins_ctas(int P, int threads, int most = INT_MAX)
+{
+    const int64_t each = (int64_t)threads * bins_items(P);
+    return (int)std::min<int64_t>(most, (P + each - 1) / each);
+}
 
 extern "C" size_t cgx_tile_bins_workspace_bytes(int W, int H)
 {
@@ -2021,15 +2041,15 @@ extern "C" int cgx_tile_bins_longest(void) { return KIND_3; }
 
 extern "C" int cgx_tile_bins_count(int P, int W, int H, const int32_t* radii, const float* means2D,
                                    const uint8_t* compute_locally, uint32_t* tiles_touched, void* workspace,
-                                   size_t workspace_bytes, uint32_t* host_words7, void* stream)
+                                   size_t workspace_bytes, uint64_t* host_words6, void* stream)
 {
     if (P <= 0 || W <= 0 || H <= 0 || !radii || !means2D || ((uintptr_t)means2D & 7) || !compute_locally ||
         !tiles_touched || !workspace || ((uintptr_t)workspace & 7))
         return CGX_EINVAL;
     if (workspace_bytes < cgx_tile_bins_workspace_bytes(W, H)) return CGX_ENOMEM;
     void* mapped = nullptr;
-    if (host_words7) {       // fails for pageable memory: the caller must pass page-locked memory
-        cudaError_t e = cudaHostGetDevicePointer(&mapped, host_words7, 0);
+    if (host_words6) {       // fails for pageable memory: the caller must pass page-locked memory
+        cudaError_t e = cudaHostGetDevicePointer(&mapped, host_words6, 0);
         if (e != cudaSuccess || !mapped) { (void)cudaGetLastError(); return CGX_EINVAL; }
     }
     const int gx = (W + CGX_BLOCK_X - 1) / CGX_BLOCK_X, gy = (H + CGX_BLOCK_Y - 1) / CGX_BLOCK_Y;
@@ -2038,17 +2058,18 @@ extern "C" int cgx_tile_bins_count(int P, int W, int H, const int32_t* radii, co
     tile_bins_carve(W, H, workspace, &b);
     tile_bins_begin_kernel<<<1, 1024, 0, st>>>(gx, gy, compute_locally, b);
     const bool vec = aligned16(radii) && aligned16(means2D) && aligned16(tiles_touched);
+    const int items = bins_items(P);
     if (bins_in_shared(P, gx * gy)) {
         const int smem = BIN_WARPS * sizeof(WarpRects) + 8 * b.eighth * sizeof(uint32_t);
         if (!allow_shared<tile_bins_count_shared_kernel>(BIN_WARPS * sizeof(WarpRects) + BIN_SHARED_TILES * sizeof(uint32_t)))
             return CGX_ECUDA;
-        tile_bins_count_shared_kernel<<<bins_shared_ctas(P), 32 * BIN_WARPS, smem, st>>>(
-            P, gx, gy, radii, (const float2*)means2D, compute_locally, tiles_touched, b, vec);
+        tile_bins_count_shared_kernel<<<bins_ctas(P, 32, BIN_CTAS), 32 * BIN_WARPS, smem, st>>>(
+            P, gx, gy, radii, (const float2*)means2D, compute_locally, tiles_touched, b, vec, items);
     } else {
-        tile_bins_count_kernel<<<(P + BIN_THREADS * BIN_ITEMS - 1) / (BIN_THREADS * BIN_ITEMS), BIN_THREADS, 0, st>>>(
-            P, gx, gy, radii, (const float2*)means2D, compute_locally, tiles_touched, b, vec);
+        tile_bins_count_kernel<<<bins_ctas(P, BIN_THREADS), BIN_THREADS, 0, st>>>(
+            P, gx, gy, radii, (const float2*)means2D, compute_locally, tiles_touched, b, vec, items);
     }
-    tile_bins_scan_kernel<<<(b.eighth + 255) / 256, 256, 0, st>>>(gx * gy, b, (volatile uint32_t*)mapped);
+    tile_bins_scan_kernel<<<(b.eighth + 255) / 256, 256, 0, st>>>(gx * gy, b, (volatile unsigned long long*)mapped);
     return check_launch(3);
 }
 
@@ -2063,18 +2084,19 @@ static int launch_tile_sort(int n_tiles, const uint32_t* tiles, const uint2* ran
 }
 
 extern "C" int cgx_tile_bins_sort(int P, int W, int H, const int32_t* radii, const float* means2D, const float* depths,
-                                  const uint8_t* compute_locally, const uint32_t* host_words7, void* workspace,
+                                  const uint8_t* compute_locally, const uint32_t* words6, void* workspace,
                                   size_t workspace_bytes, uint64_t* pairs, uint32_t* point_list, void* stream)
 {
     if (P <= 0 || W <= 0 || H <= 0 || !radii || !means2D || ((uintptr_t)means2D & 7) || !depths || !compute_locally ||
-        !host_words7 || !workspace || ((uintptr_t)workspace & 7))
+        !words6 || !workspace || ((uintptr_t)workspace & 7))
         return CGX_EINVAL;
     if (workspace_bytes < cgx_tile_bins_workspace_bytes(W, H)) return CGX_ENOMEM;
-    const uint32_t R = host_words7[0];
+    const uint32_t R = words6[0];
     if (R == 0) return CGX_OK;
     if (!pairs || !point_list) return CGX_EINVAL;
-    if (host_words7[1] > (uint32_t)KIND_3) return CGX_ENOMEM;
+    if (words6[1] > (uint32_t)KIND_3) return CGX_ENOMEM;
     const int gx = (W + CGX_BLOCK_X - 1) / CGX_BLOCK_X, gy = (H + CGX_BLOCK_Y - 1) / CGX_BLOCK_Y, T = gx * gy;
+    const int items = bins_items(P);
     cudaStream_t st = (cudaStream_t)stream;
     TileBins b;
     tile_bins_carve(W, H, workspace, &b);
@@ -2083,15 +2105,15 @@ extern "C" int cgx_tile_bins_sort(int P, int W, int H, const int32_t* radii, con
         const int smem = sizeof(BinWarps) + 8 * b.eighth * sizeof(uint32_t);
         if (!allow_shared<tile_bins_fill_shared_kernel>(sizeof(BinWarps) + BIN_SHARED_TILES * sizeof(uint32_t)))
             return CGX_ECUDA;
-        tile_bins_fill_shared_kernel<<<bins_shared_ctas(P), 32 * BIN_WARPS, smem, st>>>(
-            P, gx, gy, radii, (const float2*)means2D, depths, compute_locally, b, pairs, R, vec);
+        tile_bins_fill_shared_kernel<<<bins_ctas(P, 32, BIN_CTAS), 32 * BIN_WARPS, smem, st>>>(
+            P, gx, gy, radii, (const float2*)means2D, depths, compute_locally, b, pairs, R, vec, items);
     } else {
-        tile_bins_fill_kernel<<<(P + BIN_THREADS * BIN_ITEMS - 1) / (BIN_THREADS * BIN_ITEMS), BIN_THREADS, 0, st>>>(
-            P, gx, gy, radii, (const float2*)means2D, depths, compute_locally, b, pairs, R, vec);
+        tile_bins_fill_kernel<<<bins_ctas(P, BIN_THREADS), BIN_THREADS, 0, st>>>(
+            P, gx, gy, radii, (const float2*)means2D, depths, compute_locally, b, pairs, R, vec, items);
     }
     int s = check_launch();
     // long stretches first: their CTAs take longest
-    const uint32_t* n = host_words7 + 2;
+    const uint32_t* n = words6 + 2;
     if (s == CGX_OK && n[3]) s = launch_tile_sort<1024, KIND_3>(n[3], b.tiles + 3 * (size_t)T, b.ranges, pairs, point_list, st);
     if (s == CGX_OK && n[2]) s = launch_tile_sort<512, KIND_2>(n[2], b.tiles + 2 * (size_t)T, b.ranges, pairs, point_list, st);
     if (s == CGX_OK && n[1]) s = launch_tile_sort<256, KIND_1>(n[1], b.tiles + T, b.ranges, pairs, point_list, st);

@@ -239,13 +239,18 @@ void report(const Stats& stats, const char* key, std::shared_ptr<EventMs> ms)
 }
 
 // ---------------------------------------------------------------------------------------------- pair counts
-// The counting stage leaves the number of pairs and what the tiles' lists look like in page-locked memory, with a flag
-// behind them that the host watches: neither a copy nor an event stands between the kernel and the launches that need them.
+// The counting stage leaves the number of pairs and what the tiles' lists look like in page-locked memory, each with a
+// flag that the host watches: neither a copy nor an event stands between the kernel and the launches that need them.
 constexpr int SLOTS = 256;
 struct Slot {
-    uint32_t word[6];          // see cgx_tile_bins_count
-    volatile uint32_t flag;
-    uint32_t pad;
+    volatile uint64_t word[6];          // see cgx_tile_bins_count
+    uint64_t pad[2];
+    bool arrived() const
+    {
+        uint64_t all = ~0ull;
+        for (int k = 0; k < 6; k++) all &= word[k];
+        return all >> 32;
+    }
 };
 Slot* slots()
 {
@@ -261,7 +266,7 @@ struct Count {
     Tensor geom;
     int slot = -1;
     cudaStream_t stream = nullptr;
-    uint32_t word[7];
+    uint32_t word[6];
     Tensor keep[3];            // a prefetched count's inputs: their addresses stay taken
 };
 std::mutex slot_lock;
@@ -292,10 +297,10 @@ Count start_count(int64_t P, int W, int H, const Tensor& means2D, const Tensor& 
     c.slot = take_slot();
     c.stream = at::cuda::getCurrentCUDAStream().stream();
     Slot& s = slots()[c.slot];
-    s.flag = 0;
+    for (int k = 0; k < 6; k++) s.word[k] = 0;
     check(L.cgx_tile_bins_count((int)P, W, H, i32(radii), f32(means2D), static_cast<uint8_t*>(local.data_ptr()),
                                 at_offset<uint32_t>(c.geom, gl.tiles_touched), at_offset<void>(c.geom, gl.bins),
-                                gl.bins_bytes, s.word, c.stream), "cgx_tile_bins_count");
+                                gl.bins_bytes, const_cast<uint64_t*>(s.word), c.stream), "cgx_tile_bins_count");
     return c;
 }
 // Waits for the count; gives the slot back.
@@ -304,16 +309,15 @@ void finish_count(Count& c)
     Slot& s = slots()[c.slot];
     const auto t0 = std::chrono::steady_clock::now();
     int spins = 0;
-    while (!s.flag) {
+    while (!s.arrived()) {
         if (++spins % 1024 == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(2)) {
             // a long queue in front of it, or an error: let the driver wait, and say so if there was one
             const cudaError_t e = cudaStreamSynchronize(c.stream);
             if (e != cudaSuccess) throw std::runtime_error(std::string("cgx_tile_bins_count: ") + cudaGetErrorString(e));
-            if (!s.flag) throw std::runtime_error("cgx_tile_bins_count: the pair count did not arrive");
+            if (!s.arrived()) throw std::runtime_error("cgx_tile_bins_count: the pair count did not arrive");
         }
     }
-    std::atomic_thread_fence(std::memory_order_acquire);
-    for (int k = 0; k < 6; k++) c.word[k] = s.word[k];
+    for (int k = 0; k < 6; k++) c.word[k] = (uint32_t)s.word[k];
     give_slot(c.slot);
     c.slot = -1;
 }

@@ -388,17 +388,17 @@ int cgx_bin_count_scan_depths(int P, int W, int H, const int32_t* radii, const f
 /* Per-tile lists without sorted keys, for hosts that do not need those: for every tile the same list as emission, sort
  * and tile_ranges leave (its Gaussians by depth bits, then index), the tiles' stretches in an order of their own, in four to eight launches.
  * cgx_tile_bins_count (P > 0) fills tiles_touched (P) and the workspace (8-byte aligned), whose first 2 T words are the
- * ranges, and posts seven words to page-locked host memory (optional): pairs, longest list, tiles of four kinds by list
- * length, and last a 1 that the caller clears before and watches after the call.  cgx_tile_bins_sort takes those words
- * back and fills pairs (scratch) and point_list, both of `pairs` elements; lists longer than cgx_tile_bins_longest()
+ * ranges, and posts six words to page-locked host memory (optional): pairs, longest list, tiles of four kinds by list
+ * length, each in the low half of a 64-bit word whose high half becomes 1 (the caller clears them before the call and
+ * watches them after it, in any order).  cgx_tile_bins_sort takes the low halves back and fills pairs (scratch) and point_list, both of `pairs` elements; lists longer than cgx_tile_bins_longest()
  * give CGX_ENOMEM (use the global sort).  A workspace serves one sort. */
 size_t cgx_tile_bins_workspace_bytes(int W, int H);
 int cgx_tile_bins_longest(void);
 int cgx_tile_bins_count(int P, int W, int H, const int32_t* radii, const float* means2D, const uint8_t* compute_locally,
-                        uint32_t* tiles_touched, void* workspace, size_t workspace_bytes, uint32_t* host_words7,
+                        uint32_t* tiles_touched, void* workspace, size_t workspace_bytes, uint64_t* host_words6,
                         void* stream);
 int cgx_tile_bins_sort(int P, int W, int H, const int32_t* radii, const float* means2D, const float* depths,
-                       const uint8_t* compute_locally, const uint32_t* host_words7, void* workspace,
+                       const uint8_t* compute_locally, const uint32_t* words6, void* workspace,
                        size_t workspace_bytes, uint64_t* pairs, uint32_t* point_list, void* stream);
 
 /* duplicateWithKeys (RAST/cuda_rasterizer/rasterizer_impl.cu:74-117): writes point_offsets u32 (P)
