@@ -91,34 +91,23 @@ class AnchorStatistics:
         self.offset_gradient_accum = torch.zeros(n_anchors * n_offsets, 1, device=device)
         self.offset_denom = torch.zeros(n_anchors * n_offsets, 1, device=device)
 
-    @torch.no_grad()
     def training_statis(self, viewspace_point_grad, opacity, update_filter, offset_selection_mask, anchor_visible_mask):
         """viewspace_point_grad: (G, >=2) gradient of the screen-space positions of the G neural Gaussians that were
         rasterised; opacity: (V * n_offsets, 1) raw opacities of the V visible anchors' slots; update_filter: (G,)
         bool, Gaussian was on screen (radii > 0); offset_selection_mask: (V * n_offsets,) bool, slot produced a
         Gaussian (G = its number of True entries); anchor_visible_mask: (N,) bool with V True entries."""
-        n_off = self.n_offsets
-        accums = (self.opacity_accum, self.anchor_demon, self.offset_gradient_accum, self.offset_denom)
-        masks = (update_filter, offset_selection_mask, anchor_visible_mask)
-        if all(_plain(t, torch.float32) for t in accums) and all(_plain(m, torch.bool) for m in masks) and \
-                _plain(opacity, torch.float32) and viewspace_point_grad.is_cuda and \
-                viewspace_point_grad.dtype == torch.float32 and viewspace_point_grad.ndim == 2 and \
-                viewspace_point_grad.shape[1] >= 2 and viewspace_point_grad.stride(1) == 1 and \
-                opacity.numel() == offset_selection_mask.numel() and anchor_visible_mask.numel() and \
-                update_filter.numel() == viewspace_point_grad.shape[0] and \
-                len({t.device for t in accums + masks + (opacity, viewspace_point_grad)}) == 1:
+        if opacity.is_cuda:
             from diff_gaussian_rasterization import _lib
 
-            l = _lib.lib()
-            N, slots = anchor_visible_mask.numel(), offset_selection_mask.numel()
-            ws = torch.empty(l.cgx_anchor_stats_workspace_bytes(N, slots), dtype=torch.uint8, device=opacity.device)
-            with torch.cuda.device(opacity.device):
-                _lib.check(l.cgx_anchor_stats(
-                    N, n_off, slots, update_filter.numel(), viewspace_point_grad.data_ptr(),
-                    max(2, viewspace_point_grad.stride(0)), opacity.data_ptr(), update_filter.data_ptr(),
-                    offset_selection_mask.data_ptr(), anchor_visible_mask.data_ptr(), *[t.data_ptr() for t in accums],
-                    ws.data_ptr(), ws.numel(), _lib.current_stream_ptr()), "cgx_anchor_stats")
-            return
+            if _lib.host().anchor_stats(self.n_offsets, self.opacity_accum, self.anchor_demon, self.offset_gradient_accum,
+                                        self.offset_denom, update_filter, offset_selection_mask, anchor_visible_mask,
+                                        viewspace_point_grad, opacity):
+                return
+        self._by_tensors(viewspace_point_grad, opacity, update_filter, offset_selection_mask, anchor_visible_mask)
+
+    @torch.no_grad()
+    def _by_tensors(self, viewspace_point_grad, opacity, update_filter, offset_selection_mask, anchor_visible_mask):
+        n_off = self.n_offsets
         avm = anchor_visible_mask.view(-1, 1)
         per_anchor = opacity.detach().reshape(-1).clamp_min(0).view(-1, n_off).sum(dim=1, keepdim=True)
         self.opacity_accum += torch.zeros_like(self.opacity_accum).masked_scatter(avm, per_anchor)

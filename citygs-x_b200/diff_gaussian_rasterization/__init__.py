@@ -145,6 +145,8 @@ class GaussianRasterizer(nn.Module):
 
     def visible_filter(self, means3D, scales=None, rotations=None, cov3D_precomp=None):
         rs = self.raster_settings
+        if _C.PROFILE is None and scales is not None and rotations is not None and cov3D_precomp is None:
+            return _lib.host().visible_filter(means3D, scales, rotations, rs)
         if scales is None:
             scales = torch.Tensor([])
         if rotations is None:
