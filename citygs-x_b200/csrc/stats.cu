@@ -36,7 +36,7 @@ densify_kernel(int P, const __grid_constant__ DensifyBatch d, float* __restrict_
     if (max_radii) max_radii[i] = largest;
 }
 
-constexpr int ANCHORS = 1024;        // anchors per CTA
+constexpr int ANCHORS = 256;         // anchors per CTA, and per warp that counts
 constexpr int SLOT_CHUNK = 4096;     // slots per partial count
 
 // Sum of n <= 4096 bytes that are 0 or 1, over the CTA's 256 threads.
@@ -83,22 +83,32 @@ anchor_count_kernel(int n_anchors, long long n_slots, int anchor_blocks, const u
                     const uint8_t* __restrict__ selected, int* __restrict__ counts)
 {
     __shared__ int s_red[8];
-    const int b = blockIdx.x;
-    int c;
-    if (b < anchor_blocks) {
-        const int start = b * ANCHORS;
-        c = count_bytes(seen + start, min(ANCHORS, n_anchors - start), s_red);
-    } else {
-        const long long start = (long long)(b - anchor_blocks) * SLOT_CHUNK;
-        c = count_bytes(selected + start, (int)min((long long)SLOT_CHUNK, n_slots - start), s_red);
+    const int count_blocks = (anchor_blocks + 7) / 8;
+    if ((int)blockIdx.x < count_blocks) {
+        const int b = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+        const int64_t first = (int64_t)b * ANCHORS;
+        int c = 0;
+        if (first + ANCHORS <= n_anchors && (reinterpret_cast<uintptr_t>(seen) & 7u) == 0) {
+            const uint2 v = __ldg(reinterpret_cast<const uint2*>(seen + first) + lane);
+            c = __popc(v.x & 0x01010101u) + __popc(v.y & 0x01010101u);
+        } else {
+            for (int64_t i = first + lane; i < min(first + ANCHORS, (int64_t)n_anchors); i += 32) c += seen[i] != 0;
+        }
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0 && b < anchor_blocks) counts[b] = c;
+        return;
     }
-    if (threadIdx.x == 0) counts[b] = c;
+    const int b = blockIdx.x - count_blocks;
+    const long long start = (long long)b * SLOT_CHUNK;
+    const int c = count_bytes(selected + start, (int)min((long long)SLOT_CHUNK, n_slots - start), s_red);
+    if (threadIdx.x == 0) counts[anchor_blocks + b] = c;
 }
 
 // Per CTA of ANCHORS anchors: its visible ones (in order) own consecutive slots, the selected among those consecutive
-// Gaussians; where both begin follows from the partial counts.  500 k anchors of ten slots: 270 -> 27 us a call
-// with the counting launch, of 34 launches and four device-wide scans.
-__global__ void __launch_bounds__(256)
+// Gaussians; where both begin follows from the partial counts.  Bound by the latency of its chains of dependent loads
+// (mask, rank, Gaussian, sum): few anchors per CTA, and a warp has 128 slots in flight.  500 k anchors of ten slots, with
+// the counting launch: 270 us (34 launches, four device-wide scans) -> 46 with 1024 anchors and 32 slots -> 34.
+__global__ void __launch_bounds__(256, 5)
 anchor_stats_kernel(int n_anchors, int n_off, long long n_slots, long long n_gaussians, int anchor_blocks,
                     const int* __restrict__ counts, const uint8_t* __restrict__ seen,
                     const uint8_t* __restrict__ selected, const uint8_t* __restrict__ on_screen,
@@ -147,6 +157,7 @@ anchor_stats_kernel(int n_anchors, int n_off, long long n_slots, long long n_gau
     for (int j = t; j < n_seen; j += 256) {
         const float* o = opacity + slot0 + (long long)j * n_off;
         float sum = 0.f;
+#pragma unroll 5
         for (int k = 0; k < n_off; k++) sum += fmaxf(o[k], 0.f);
         const int a = a0 + s_anchor[j];
         opacity_accum[a] += sum;
@@ -162,23 +173,44 @@ anchor_stats_kernel(int n_anchors, int n_off, long long n_slots, long long n_gau
     __syncthreads();
     if (lane == 0) s_red[warp] = chosen;
     __syncthreads();
-    long long rank = g0;
+    int rank = 0;                                  // from the CTA's first Gaussian
 #pragma unroll
     for (int w = 0; w < 8; w++)
         if (w < warp) rank += s_red[w];
-    for (int s0 = s_begin; s0 < s_end; s0 += 32) {
-        const int s = s0 + lane;
-        const bool sel = s < s_end && selected[slot0 + s];
-        const uint32_t sm = __ballot_sync(0xffffffffu, sel);
-        const long long g = rank + __popc(sm & ((1u << lane) - 1u));
-        rank += __popc(sm);
-        if (sel && g < n_gaussians && on_screen[g]) {
-            const float x = grad[g * grad_stride], y = grad[g * grad_stride + 1];
-            const int j = s / n_off;
-            const long long to = (long long)(a0 + s_anchor[j]) * n_off + (s - j * n_off);
-            gradient_accum[to] += sqrtf(x * x + y * y);
-            denom[to] += 1.f;
+    constexpr int FLIGHT = 4;
+    on_screen += g0;
+    grad += g0 * grad_stride;
+    gradient_accum += (long long)a0 * n_off;
+    denom += (long long)a0 * n_off;
+    const int here = (int)max(0ll, min(n_gaussians - g0, (long long)slots));
+    for (int s0 = s_begin; s0 < s_end; s0 += 32 * FLIGHT) {
+        bool sel[FLIGHT], seen_g[FLIGHT];
+        int to[FLIGHT];
+        float x[FLIGHT], y[FLIGHT], sum[FLIGHT], visits[FLIGHT];
+#pragma unroll
+        for (int f = 0; f < FLIGHT; f++) {
+            const int s = s0 + 32 * f + lane;
+            sel[f] = s < s_end && selected[slot0 + s];
         }
+#pragma unroll
+        for (int f = 0; f < FLIGHT; f++) {
+            const uint32_t sm = __ballot_sync(0xffffffffu, sel[f]);
+            const int g = rank + __popc(sm & ((1u << lane) - 1u));
+            rank += __popc(sm);
+            sel[f] = sel[f] && g < here;
+            if (!sel[f]) continue;
+            const int s = s0 + 32 * f + lane, j = s / n_off;
+            to[f] = s_anchor[j] * n_off + (s - j * n_off);
+            seen_g[f] = on_screen[g];
+            x[f] = grad[(long long)g * grad_stride], y[f] = grad[(long long)g * grad_stride + 1];
+            sum[f] = gradient_accum[to[f]], visits[f] = denom[to[f]];
+        }
+#pragma unroll
+        for (int f = 0; f < FLIGHT; f++)
+            if (sel[f] && seen_g[f]) {
+                gradient_accum[to[f]] = sum[f] + sqrtf(x[f] * x[f] + y[f] * y[f]);
+                denom[to[f]] = visits[f] + 1.f;
+            }
     }
 }
 
@@ -223,7 +255,7 @@ extern "C" int cgx_anchor_stats(int n_anchors, int n_offsets, int64_t n_slots, i
     const int anchor_blocks = (n_anchors + ANCHORS - 1) / ANCHORS;
     const int slot_blocks = (int)((n_slots + SLOT_CHUNK - 1) / SLOT_CHUNK);
     cudaStream_t st = (cudaStream_t)stream;
-    anchor_count_kernel<<<anchor_blocks + slot_blocks, 256, 0, st>>>(n_anchors, n_slots, anchor_blocks, seen, selected,
+    anchor_count_kernel<<<(anchor_blocks + 7) / 8 + slot_blocks, 256, 0, st>>>(n_anchors, n_slots, anchor_blocks, seen, selected,
                                                                      (int*)workspace);
     anchor_stats_kernel<<<anchor_blocks, 256, 0, st>>>(n_anchors, n_offsets, n_slots, n_gaussians, anchor_blocks,
                                                        (const int*)workspace, seen, selected, on_screen, opacity, grad,

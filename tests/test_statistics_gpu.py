@@ -8,7 +8,7 @@ import util  # noqa: F401
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("N,n_off,seen,sel", [(1, 1, 1.0, 1.0), (1023, 10, 0.5, 0.6), (1024, 4, 1.0, 1.0),
+@pytest.mark.parametrize("N,n_off,seen,sel", [(1, 1, 1.0, 1.0), (255, 10, 0.9, 0.9), (256, 3, 1.0, 0.5), (2049, 10, 0.3, 0.6), (1023, 10, 0.5, 0.6), (1024, 4, 1.0, 1.0),
                                               (1025, 4, 0.02, 0.5), (5000, 7, 0.9, 0.1), (20000, 10, 0.3, 0.6),
                                               (3000, 5, 0.0, 0.5)])
 def test_anchor_statistics(N, n_off, seen, sel, cuda_device):
